@@ -93,6 +93,33 @@ def test_small_shapes_match_oracle(A, shape):
     _against_oracle(A, p)
 
 
+@pytest.mark.parametrize("nz", [3, 31, 32, 41, 64, 81, 82, 128])  # either side of each tile width
+@pytest.mark.parametrize("method", [AI.REMAP_PLM, AI.REMAP_PPM])
+@pytest.mark.parametrize("n_passive", [-1, 0, 1])  # one, two and three tracers
+def test_tile_edges_and_serial_columns(A, nz, method, n_passive):
+    """Ragged last tiles, odd tracer counts, and columns that take the serial sweep: negative or NaN
+    thicknesses, averages that are infinite or NaN."""
+    p = AI.random_case(9, 5, nz, 1100 + nz, method=method, n_passive=max(n_passive, 0), conserve_ke=nz % 2 == 1)
+    if n_passive < 0:
+        p.tracers, p.idx_salinity = p.tracers[:1], -1
+    p.h_layer[nz // 2, 1, 2] = -0.5
+    p.h_layer[0, 3, 7] = np.nan
+    p.h_layer[nz - 1, 2, 4] = 500.0
+    p.tracers[0][nz - 1, 2, 4] = np.inf
+    p.tracers[-1][0, 4, 8] = np.nan
+    p.h_layer[0, 4, 8] = 100.0
+    p.u[nz - 1, 0, 3] = np.nan
+    p.v[1, 2, 0] = -np.inf
+    d, q = A.to_device(p), p.copy()
+    A.step_problem(p, d, 1)
+    with np.errstate(all="ignore"):
+        AO.step(q, 1)
+    torch.cuda.synchronize()
+    got, want = A.host_arrays(d), q.arrays()
+    for k in want:
+        assert np.array_equal(got[k], want[k], equal_nan=True), k
+
+
 def test_many_tracers_absent_slots_no_faces(A):
     """11 slots (two launches of tracers), two of them unallocated, no face velocities."""
     p = AI.random_case(19, 15, 10, 801, n_passive=9, faces=False, name="many")
