@@ -231,15 +231,17 @@ REDI_B200_API int redi_b200_eos_points(const redi_b200_eos* eos, int n, const do
                                        const double* p, double* rho, double* dsv_dt, double* dsv_ds, void* stream);
 
 /* Largest number of tracers whose face fluxes one launch computes (1, 2, 4
- * or 8; default 8), process-wide (no counterpart in the reference). Larger
+ * or 8; default 2), process-wide (no counterpart in the reference). Larger
  * groups read the Phase-A coefficients fewer times per step, smaller ones run
  * at higher occupancy; results do not depend on it. */
 REDI_B200_API int redi_b200_set_tracer_group(int max_group);
 REDI_B200_API int redi_b200_get_tracer_group(void);
 
 /* Tracers one cell-gather launch folds (2, 4 or 8; default 2) and where it
- * keeps a chunk's per-layer sums (smem = 1, the default: the thread's slots in
- * shared memory, one load-add-store per flux; 2: the same, fetching 8
+ * walks (smem = 4, the default: a warp on whole rows of sublayers, in pairs of
+ * tracers and chunks of its own, sums in shared memory; the others let each
+ * thread walk at its own pace and differ in where a chunk's per-layer sums
+ * live: 1: the thread's slots in shared memory, one load-add-store per flux; 2: the same, fetching 8
  * sublayers per round trip instead of 3 or 4; 3: the same with batches of 4
  * software-pipelined, the next batch in flight while one is folded; 0:
  * registers, a select-add over the chunk), process-wide (no counterpart in the

@@ -279,9 +279,12 @@ Profiler g_prof;
 namespace redi {
 void set_last_error(const std::string& msg) { g_last_error = msg; }
 
-// the autotuner's usual gather choice at config 1; the sweep's windows in a
-// shared-memory ring of 4 interfaces
-static CellTuning g_cell_tuning{64, 2, 8, 8, 2, 1, 0, 0, 4};
+// the row gather; the shape the other gather forms take when one is chosen;
+// face fluxes of two tracers per launch (720x576x50 mixed, 32 passive tracers:
+// groups of 2 15.4 ms, 4 20.0, 8 28.7; 361x275x51 FP64, 5 tracers: 1.34 and
+// 1.97 ms: the larger groups' registers cost more residency than the shared
+// coefficient reads save); the sweep's windows in a shared-memory ring of 4
+static CellTuning g_cell_tuning{64, 2, 8, 2, 2, 1, 0, 0, 4, 0, 1};
 CellTuning cell_tuning() { return g_cell_tuning; }
 void set_cell_tuning(const CellTuning& t) { g_cell_tuning = t; }
 static FoldTuning g_fold_tuning{0, 2, 0, 0, 0};  // the pair stays the default until the fused pass is faster
@@ -403,12 +406,13 @@ int redi_b200_get_tracer_group(void) { return redi::cell_tuning().group; }
 
 int redi_b200_set_gather_tracers(int n, int smem) {
     if (n != 2 && n != 4 && n != 8) return fail(REDI_B200_E_ARG, "redi_b200_set_gather_tracers: n must be 2, 4 or 8");
-    if (smem < 0 || smem > 3) return fail(REDI_B200_E_ARG, "redi_b200_set_gather_tracers: smem must be 0, 1, 2 or 3");
+    if (smem < 0 || smem > 4) return fail(REDI_B200_E_ARG, "redi_b200_set_gather_tracers: smem must be 0, 1, 2, 3 or 4");
     redi::CellTuning t = redi::cell_tuning();
     t.gather_tracers = n;
     t.gather_smem = smem ? 1 : 0;
     t.gather_batch = smem == 2 ? 8 : 0;
     t.gather_pipe = smem == 3 ? 1 : 0;
+    t.gather_rows = smem == 4 ? 1 : 0;
     redi::set_cell_tuning(t);
     return REDI_B200_OK;
 }
@@ -437,7 +441,7 @@ int redi_b200_get_sweep_form(void) { return redi::cell_tuning().sweep_form; }
 
 int redi_b200_get_gather_tracers(int* smem) {
     const redi::CellTuning t = redi::cell_tuning();
-    if (smem) *smem = t.gather_smem ? (t.gather_pipe ? 3 : (t.gather_batch >= 8 ? 2 : 1)) : 0;
+    if (smem) *smem = t.gather_rows ? 4 : t.gather_smem ? (t.gather_pipe ? 3 : (t.gather_batch >= 8 ? 2 : 1)) : 0;
     return redi::cell_tuning().gather_tracers;
 }
 

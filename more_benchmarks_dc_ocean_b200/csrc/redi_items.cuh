@@ -2024,5 +2024,206 @@ __device__ __forceinline__ void gather_item_s(const CellGatherArgsT<P>& a, int i
     if (bad && a.err) atomicAdd(a.err, bad);
 }
 
+// ---------------------------------------------------------------------------
+// The fold with every lane of a warp on the same sublayer.
+//
+// In gather_run_s each lane continues where its own chunk ended, so the lanes
+// of a warp read different sublayers at a time, and a 32-byte sector of the
+// flux and Ko rows is fetched for 8 or 4 of its bytes. Here a warp starts a
+// chunk at the first sublayer any of its lanes still needs and reads whole
+// rows, U of them ahead of the U it adds; a lane adds nothing before its own
+// first sublayer and after its last. The sums (shared memory, this warp's:
+// [CH + 2][32][NT], row 0 and row CH + 1 take those idle additions) of a batch
+// are read together, a run of one layer is carried in registers (one addition
+// per sublayer in the chain instead of a shared-memory round trip) and each is
+// written back: exactly the additions of gather_run, in its order, as long as
+// the layers of a batch do not decrease; a batch in which they do (not possible
+// for sweep-produced coefficients) is added one by one.
+// ---------------------------------------------------------------------------
+constexpr int kGatherRowThreads = 32;
+
+template <int NT>
+struct alignas(NT * sizeof(double)) LaneSums {
+    double v[NT];
+};
+template <int NT>
+__device__ __forceinline__ LaneSums<NT> ld_sums(const char* p) {
+    LaneSums<NT> r;
+    if constexpr (NT == 2) {
+        const double2 d = *reinterpret_cast<const double2*>(p);
+        r.v[0] = d.x;
+        r.v[1] = d.y;
+    } else {
+        r.v[0] = *reinterpret_cast<const double*>(p);
+    }
+    return r;
+}
+template <int NT>
+__device__ __forceinline__ void st_sums(char* p, const LaneSums<NT>& r) {
+    if constexpr (NT == 2) *reinterpret_cast<double2*>(p) = make_double2(r.v[0], r.v[1]);
+    else *reinterpret_cast<double*>(p) = r.v[0];
+}
+
+// One face's sublayers of the chunk [k0, k0 + ch) from sublayer s on (the same
+// for the whole warp); `on`: this lane has the face. first: the lane's first
+// sublayer not yet added. Returns the next chunk's s. Every lane must call it.
+// The left face's column gains its fluxes, the right one's loses them: `sign`
+// is the sign bit to flip, an addition of -f being the subtraction of f.
+__device__ __forceinline__ double flip(double f, int sign) {
+    return __hiloint2double(__double2hiint(f) ^ sign, __double2loint(f));
+}
+template <int NT, class P, class LD, int U>
+__device__ __forceinline__ int gather_walk_rows(const typename P::Flux* __restrict__ F, unsigned f_stride,
+                                                const typename P::Ko* __restrict__ KoS, unsigned fo, unsigned stride,
+                                                int ns1, bool on, int sign, int s, int& first, int k0, int ch,
+                                                char* __restrict__ acc, int& bad) {
+    constexpr int kRow = kGatherRowThreads * NT * (int)sizeof(double);
+    int kk[U];
+    typename P::Flux ff[U][NT];
+    auto fetch = [&](int s0, int (&k)[U], typename P::Flux (&f)[U][NT]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const unsigned x = (unsigned)min(s0 + u, ns1 - 1) * stride + fo;
+            k[u] = (int)LD::ld(KoS + x);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) f[u][n] = LD::ld(F + (size_t)n * f_stride + x);
+        }
+    };
+    bool stop = !on;
+    int next = on ? first : ns1;
+    if (on) fetch(s, kk, ff);
+    while (s < ns1) {
+        int kn[U];
+        typename P::Flux fn[U][NT];
+        if (on) fetch(s + U, kn, fn);
+        int row[U];
+        bool ordered = true;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool wait = s + u < first;
+            stop = stop || (!wait && (kk[u] >= k0 + ch || s + u >= ns1));
+            next += !stop && !wait ? 1 : 0;
+            row[u] = stop ? ch + 1 : (wait ? 0 : kk[u] - k0 + 1);
+            if (row[u] < 1 && !wait) {  // a layer above the chunk
+                ++bad;
+                row[u] = 0;
+            }
+            if (u) ordered = ordered && row[u] >= row[u - 1];
+        }
+        if (on && ordered) {
+            LaneSums<NT> v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = ld_sums<NT>(acc + row[u] * kRow);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bool same = u && row[u] == row[u ? u - 1 : 0];
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    const double b = same ? v[u ? u - 1 : 0].v[n] : v[u].v[n];
+                    v[u].v[n] = b + flip((double)ff[u][n], sign);
+                }
+                st_sums<NT>(acc + row[u] * kRow, v[u]);
+            }
+        } else if (on) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                LaneSums<NT> v = ld_sums<NT>(acc + row[u] * kRow);
+#pragma unroll
+                for (int n = 0; n < NT; ++n) v.v[n] = v.v[n] + flip((double)ff[u][n], sign);
+                st_sums<NT>(acc + row[u] * kRow, v);
+            }
+        }
+        if (__all_sync(0xffffffffu, stop)) break;
+        s += U;
+        if (on) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                kk[u] = kn[u];
+#pragma unroll
+                for (int n = 0; n < NT; ++n) ff[u][n] = fn[u][n];
+            }
+        }
+    }
+    first = next;
+    return __reduce_min_sync(0xffffffffu, next);
+}
+
+// Cell col (col < c1: this lane has one) for the tracers tr0 .. tr0+NT-1, all
+// of the state's, whose fluxes sit at slots fslot .. fslot+NT-1; ch layers per chunk.
+template <int NT, class P, class LD, int U>
+__device__ __forceinline__ void gather_item_rows(const CellGatherArgsT<P>& a, int col, int c1, int tr0, int fslot,
+                                                 int ch, char* __restrict__ acc, int2* __restrict__ walk) {
+    constexpr int kRow = kGatherRowThreads * NT * (int)sizeof(double);
+    const bool mine = col < c1;
+    if (!mine) col = c1 - 1;
+    const int nx = a.nx, ny = a.ny, nz = a.nz, ns1 = 2 * nz + 1;
+    const size_t ncol = (size_t)nx * ny;
+    const int j = col / nx, i = col - nx * j;
+    const int I = i + 1, J = j + 1;  // Fortran indices
+    const int wuf_w = a.nghost + 1, wuf_e = a.nghost + a.nxp + 1;
+    const int wvf_s = a.nghost + 1, wvf_n = a.nghost + a.nyp + 1;
+    const unsigned ustride = (unsigned)(nx + 1) * ny, vstride = (unsigned)nx * (ny + 1);
+    bool on[4] = {mine && I >= 2 && !((a.wall_w && I == wuf_w) || (a.wall_e && I == wuf_e)),
+                  mine && I <= nx - 1 && !((a.wall_w && I + 1 == wuf_w) || (a.wall_e && I + 1 == wuf_e)),
+                  mine && J >= 2 && !((a.wall_s && J == wvf_s) || (a.wall_n && J == wvf_n)),
+                  mine && J <= ny - 1 && !((a.wall_s && J + 1 == wvf_s) || (a.wall_n && J + 1 == wvf_n))};
+    const int fo[4] = {i + (nx + 1) * j, i + 1 + (nx + 1) * j, i + nx * j, i + nx * (j + 1)};
+    if (a.u.dry) {  // dry faces carry only +0.0 fluxes
+        on[0] = on[0] && !LD::ld(a.u.dry + fo[0]);
+        on[1] = on[1] && !LD::ld(a.u.dry + fo[1]);
+    }
+    if (a.v.dry) {
+        on[2] = on[2] && !LD::ld(a.v.dry + fo[2]);
+        on[3] = on[3] && !LD::ld(a.v.dry + fo[3]);
+    }
+    const int onm = (on[0] ? 1 : 0) | (on[1] ? 2 : 0) | (on[2] ? 4 : 0) | (on[3] ? 8 : 0);
+    const double iaij = 1.0 / LD::ld(a.areaT + col);
+    const size_t su = (size_t)fslot * ns1 * ustride, sv = (size_t)fslot * ns1 * vstride;
+    const unsigned fu = (unsigned)ns1 * ustride, fv = (unsigned)ns1 * vstride;
+    int bad = 0;
+    for (int f = 0; f < 4; ++f) walk[f * kGatherRowThreads] = make_int2(0, 0);
+    for (int k0 = 1; k0 <= nz; k0 += ch) {
+        const int n = min(ch, nz + 1 - k0);
+        for (int x = 0; x <= n + 1; ++x) st_sums<NT>(acc + x * kRow, LaneSums<NT>{});
+        // one copy of the walk for the four faces (W, E, S, N): unrolled, its loads in flight exceed the registers
+#pragma unroll 1
+        for (int f = 0; f < 4; ++f) {
+            const bool left = (f & 1) != 0, isu = f < 2;
+            const bool o = (onm >> f) & 1;
+            int2 w = walk[f * kGatherRowThreads];
+            const unsigned x = isu ? i + (nx + 1) * j + (left ? 1 : 0) : i + nx * (j + (left ? 1 : 0));
+            const typename P::Ko* K = isu ? (left ? a.u.KoL : a.u.KoR) : (left ? a.v.KoL : a.v.KoR);
+            w.x = gather_walk_rows<NT, P, LD, U>(isu ? a.Fu + su : a.Fv + sv, isu ? fu : fv, K, x,
+                                                 isu ? ustride : vstride, ns1, o, left ? 0 : (int)0x80000000, w.x, w.y,
+                                                 k0, n, acc, bad);
+            walk[f * kGatherRowThreads] = w;
+        }
+        // layers k0 .. k0+n-1 are complete: hTr(knat) += dTr(knat) * (1/areaT), knat = nz + 1 - k
+        if (mine) {
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                double* out = a.htr[tr0 + t] + col;
+                const double* in = a.htr_in[tr0 + t] + col;
+                constexpr int B = 8;
+                for (int x0 = 0; x0 < n; x0 += B) {  // a batch's loads before its stores (out may be in)
+                    double x[B];
+#pragma unroll
+                    for (int b = 0; b < B; ++b)
+                        if (x0 + b < n) x[b] = in[(size_t)(nz - k0 - x0 - b) * ncol];
+#pragma unroll
+                    for (int b = 0; b < B; ++b)
+                        if (x0 + b < n)
+                            out[(size_t)(nz - k0 - x0 - b) * ncol] =
+                                x[b] + ld_sums<NT>(acc + (x0 + b + 1) * kRow).v[t] * iaij;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+        if (((onm >> f) & 1) && walk[f * kGatherRowThreads].y < ns1) ++bad;  // fluxes whose cell-side layer is beyond nz
+    if (bad && a.err) atomicAdd(a.err, bad);
+}
+
 }  // namespace plain
 }  // namespace redi

@@ -228,6 +228,7 @@ struct CellTuning {
     int gather_batch = 0;  // shared-memory gather: sublayers per round trip (8, or 0: 3 / 4 by chunk)
     int sweep_form = 4;    // neutral sweep: 0 register windows, 3 / 4 / 5 windows in a shared-memory ring of that size
     int gather_pipe = 0;   // shared-memory gather: batches of 4 software-pipelined (the next one in flight)
+    int gather_rows = 0;   // the gather with a warp on whole rows of sublayers, in pairs of tracers
 };
 CellTuning cell_tuning();
 void set_cell_tuning(const CellTuning& t);
@@ -241,7 +242,7 @@ inline int flux_group(int ntr, const CellTuning& t) {
 // Whether one gather folds the fluxes of two face-flux launches of 4 tracers
 // (8 tracers per gather: the shared-memory gather with 4-layer chunks).
 inline bool gather_spans_two(int ntr, const CellTuning& t) {
-    return t.gather_tracers >= 8 && flux_group(ntr, t) == 4 && ntr > 4 && t.gather_smem && t.chunk == 4 &&
+    return !t.gather_rows && t.gather_tracers >= 8 && flux_group(ntr, t) == 4 && ntr > 4 && t.gather_smem && t.chunk == 4 &&
            t.bx * t.by == 128;
 }
 // Slots of the flux buffer Phase B needs for ntr tracers.

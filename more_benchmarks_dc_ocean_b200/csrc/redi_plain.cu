@@ -158,6 +158,17 @@ __global__ void __launch_bounds__(kGatherThreads) k_cell_gather_s(CellGatherArgs
         gather_item_s<NT, CH, P, LdNC, kU, PIPE>(a, blockIdx.x * blockDim.x + threadIdx.x, j, tr0, fslot, acc + tid);
 }
 
+// The gather with a warp on whole rows of sublayers (gather_item_rows): one
+// warp per block, cells [c0, c1) in column order, so a ragged nx wastes no lane.
+template <int NT, class P, int U>
+__global__ void __launch_bounds__(kGatherRowThreads) k_cell_gather_rows(CellGatherArgsT<P> a, int tr0, int fslot, int c0,
+                                                                        int c1, int ch) {
+    extern __shared__ __align__(16) char rowsum[];
+    __shared__ int2 walk[4 * kGatherRowThreads];  // per face: the warp's and the lane's next sublayer
+    gather_item_rows<NT, P, LdNC, U>(a, c0 + blockIdx.x * kGatherRowThreads + threadIdx.x, c1, tr0, fslot, ch,
+                                     rowsum + threadIdx.x * NT * sizeof(double), walk + threadIdx.x);
+}
+
 // The point EOS at n independent points, as the column state evaluates it at
 // each interface (eos_density_point + eos_specvol_derivs).
 __global__ void __launch_bounds__(128) k_eos_points(EosParams e, int n, const double* __restrict__ T,
@@ -276,6 +287,34 @@ cudaError_t launch_sweep(const SweepArgsT<P>& sw, cudaStream_t st, Band band) {
     return cudaGetLastError();
 }
 
+// The row gather's batch and largest chunk. A block is one warp; registers
+// (220 FP64, 168 mixed) admit 9 and 12 of them per SM, and the chunk's sums are
+// sized to leave them an L1 that holds their rows in flight. Gather time at
+// 1440x1080x75 FP64, 2 tracers, batches of 8: chunks of 13 3.90 ms, 19 3.65,
+// 25 3.44, 38 (7 warps by shared memory) 4.53; batches of 4, 25 layers: 4.57;
+// one tracer per pass, 38 layers: 3.84; the thread-paced walk (gather_run_s):
+// 4.85. 720x576x50 mixed, 34 tracers: batches of 6, chunks of 17 9.46 ms, 25
+// 10.62; batches of 8, 17 11.57; the thread-paced walk's best 11.47. A nz up
+// to the bound is one chunk (128x96x25: 0.040 ms; 13 layers 0.047), a larger one is cut evenly.
+template <class P>
+struct RowGather {
+    static constexpr int kBatch = P::kMixed ? 6 : 8;
+    static constexpr int kChunk = P::kMixed ? 19 : 25;
+};
+
+template <int NT, class P>
+static void launch_gather_rows(const CellGatherArgsT<P>& cg, int tr, int slot, const BandRanges& r, cudaStream_t st) {
+    using G = RowGather<P>;
+    const int chunks = (cg.nz + G::kChunk - 1) / G::kChunk, ch = (cg.nz + chunks - 1) / chunks;
+    const size_t smem = (size_t)(ch + 2) * NT * plain::kGatherRowThreads * sizeof(double);
+    const int c0 = r.j0 * cg.nx, c1 = r.j1 * cg.nx;
+    launch_begin(K_CELL_UPDATE, st);
+    plain::k_cell_gather_rows<NT, P, G::kBatch>
+        <<<(unsigned)((c1 - c0 + plain::kGatherRowThreads - 1) / plain::kGatherRowThreads), plain::kGatherRowThreads,
+           smem, st>>>(cg, tr, slot, c0, c1, ch);
+    launch_end(K_CELL_UPDATE, st);
+}
+
 template <int GNT, class P>
 static void launch_gather(const CellGatherArgsT<P>& cg, int tr, int slot, const BandRanges& r, const CellTuning& tune,
                           dim3 cgrid, dim3 block, cudaStream_t st) {
@@ -387,6 +426,13 @@ static void launch_gathers(const CellGatherArgsT<P>& cg, int tr0, const BandRang
     const dim3 block(tune.bx, tune.by);
     const dim3 cgrid((cg.nx + tune.bx - 1) / tune.bx, (r.j1 - r.j0 + tune.by - 1) / tune.by);
     if (cgrid.y == 0) return;
+    if (tune.gather_rows) {  // pairs; an odd last tracer, or a flux buffer of one slot, alone
+        for (int g = 0; g < NS && tr0 + g < cg.ntr; g += 2) {
+            if (g + 1 < NS && tr0 + g + 1 < cg.ntr) launch_gather_rows<2, P>(cg, tr0 + g, g, r, st);
+            else launch_gather_rows<1, P>(cg, tr0 + g, g, r, st);
+        }
+        return;
+    }
     if constexpr (WIDE) {
         launch_gather_8<P>(cg, tr0, r, tune, cgrid, block, st);
         return;

@@ -306,6 +306,28 @@ def test_gather_forms_match_oracle(redi_lib, oracle_lib, gnt, smem, chunk):
         autotune.set_tracer_group(saved[2])
 
 
+@pytest.mark.parametrize("nx,ny,nz,npas,group", [(45, 27, 19, 3, 2), (33, 31, 25, 0, 2), (30, 21, 26, 1, 2),
+                                                 (31, 9, 51, 0, 1), (64, 20, 1, 0, 2), (29, 12, 3, 6, 8),
+                                                 (13, 40, 20, 2, 4)])
+def test_row_gather_matches_oracle(redi_lib, oracle_lib, nx, ny, nz, npas, group):
+    """The row gather at one chunk, a chunk's bound and one past it, odd tracer counts, ragged warps
+    and each size of the flux buffer: the reference's additions in its order, so the oracle's bits."""
+    from more_benchmarks_dc_ocean_b200 import autotune
+
+    saved = (autotune.get_gather_tracers(), autotune.get_tracer_group())
+    try:
+        autotune.set_gather_tracers(2, 4)
+        autotune.set_tracer_group(group)
+        p = inputs.make_problem(nx, ny, nz, n_passive=npas, seed=nx)
+        _, tg = _run_gpu(p, 1, redi_lib, check_coeffs=False)
+        _, to = _run_oracle(p, 1)
+        for n, (a, b) in enumerate(zip(tg, to)):
+            _assert_exact(f"row gather {nx}x{ny}x{nz} group={group} tracer {n}", a, b)
+    finally:
+        autotune.set_gather_tracers(*saved[0])
+        autotune.set_tracer_group(saved[1])
+
+
 @pytest.mark.parametrize("form,group,precision", [(1, 1, 0), (1, 2, 0), (1, 2, 1), (2, 1, 0), (2, 2, 0), (2, 4, 0),
                                                    (2, 2, 1), (2, 4, 1)])
 def test_staged_face_flux_matches(redi_lib, oracle_lib, form, group, precision):
