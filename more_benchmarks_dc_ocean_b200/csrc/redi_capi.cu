@@ -143,47 +143,67 @@ struct PhaseBInputs {
     redi::FaceInT<P> u, v;
 };
 
+// Phase B's buffers in the scratch for a batch of nt tracers out of ntr.
+template <class P>
+struct PhaseBBuffers {
+    int batch, group;
+    size_t recon, flux;
+    PhaseBBuffers(int nx, int ny, int nz, int ntr)
+        : batch(ntr < redi::kMaxTracers ? ntr : redi::kMaxTracers),
+          group(redi::flux_slots(batch, redi::cell_tuning())),
+          recon(redi::recon_bytes<P>(nx, ny, nz, batch)),
+          flux(redi::flux_bytes<P>(nx, ny, nz, group)) {}
+};
+
+// The face-flux arguments of a batch of nt tracers over those buffers.
+template <class P>
+redi::FaceFluxArgsT<P> flux_args(const PhaseBInputs<P>& in, const PhaseBBuffers<P>& buf, int nt, const Scratch& ws) {
+    using Flux = typename P::Flux;
+    char* base = static_cast<char*>(ws.data());
+    redi::FaceFluxArgsT<P> ff{};
+    ff.nx = in.nx; ff.ny = in.ny; ff.nz = in.nz; ff.ntr = nt;
+    ff.nghost = in.nghost; ff.nxp = in.nxp; ff.nyp = in.nyp;
+    ff.wall_w = in.walls[0]; ff.wall_e = in.walls[1]; ff.wall_s = in.walls[2]; ff.wall_n = in.walls[3];
+    ff.dt = in.dt; ff.khtr = in.khtr; ff.khtr_u = in.khtr_u; ff.khtr_v = in.khtr_v;
+    ff.dy_cu = in.dy_cu; ff.dx_cv = in.dx_cv; ff.idxCu = in.idxCu; ff.idyCv = in.idyCv;
+    ff.u = in.u; ff.v = in.v;
+    ff.ti = reinterpret_cast<double*>(base);
+    ff.ppm = reinterpret_cast<typename P::Ppm*>(base + redi::recon_ppm_offset(in.nx, in.ny, in.nz, nt));
+    ff.Fu = reinterpret_cast<Flux*>(base + buf.recon);
+    ff.Fv = ff.Fu + (size_t)buf.group * (size_t)(2 * in.nz + 1) * (size_t)(in.nx + 1) * in.ny;
+    return ff;
+}
+
 // htr_in (may be null: in place) holds the pre-step tracers, htr receives the
-// updated ones; band restricts the launches to a band of rows.
+// updated ones; band restricts the launches to a band of rows. recon_from and
+// flux_from: tracers of the first batch already reconstructed, and with their
+// fluxes already in the buffer.
 template <class P>
 int run_phase_b(const PhaseBInputs<P>& in, int ntr, double* const* htr, Scratch& ws, cudaStream_t st,
-                const double* const* htr_in = nullptr, redi::Band band = redi::Band{}, int recon_from = 0) {
-    const int batch = ntr < redi::kMaxTracers ? ntr : redi::kMaxTracers;
-    const size_t recon = redi::recon_bytes<P>(in.nx, in.ny, in.nz, batch);
-    const int group = redi::flux_slots(batch, redi::cell_tuning());
-    const size_t flux = redi::flux_bytes<P>(in.nx, in.ny, in.nz, group);
-    cudaError_t e = ws.reserve(recon + flux);
+                const double* const* htr_in = nullptr, redi::Band band = redi::Band{}, int recon_from = 0,
+                int flux_from = 0) {
+    const PhaseBBuffers<P> buf(in.nx, in.ny, in.nz, ntr);
+    cudaError_t e = ws.reserve(buf.recon + buf.flux);
     if (e != cudaSuccess) return cuda_fail(e, "scratch allocation (phase B)");
-    const size_t ns1 = (size_t)(2 * in.nz + 1);
-    using Flux = typename P::Flux;
-    Flux* Fu = reinterpret_cast<Flux*>(static_cast<char*>(ws.data()) + recon);
-    Flux* Fv = Fu + (size_t)group * ns1 * (size_t)(in.nx + 1) * in.ny;
-    for (int t0 = 0; t0 < ntr; t0 += batch) {
-        const int nt = (ntr - t0) < batch ? (ntr - t0) : batch;
+    for (int t0 = 0; t0 < ntr; t0 += buf.batch) {
+        const int nt = (ntr - t0) < buf.batch ? (ntr - t0) : buf.batch;
+        const redi::FaceFluxArgsT<P> ff = flux_args(in, buf, nt, ws);
         redi::ReconArgsT<P> rc{};
         rc.nx = in.nx; rc.ny = in.ny; rc.nz = in.nz; rc.ntr = nt; rc.h = in.h;
-        rc.ti = reinterpret_cast<double*>(ws.data());
-        rc.ppm = reinterpret_cast<typename P::Ppm*>(static_cast<char*>(ws.data()) +
-                                                    redi::recon_ppm_offset(in.nx, in.ny, in.nz, nt));
+        rc.ti = const_cast<double*>(ff.ti);
+        rc.ppm = const_cast<typename P::Ppm*>(ff.ppm);
         rc.dry_u = in.u.dry; rc.dry_v = in.v.dry;
-        redi::FaceFluxArgsT<P> ff{};
-        ff.nx = in.nx; ff.ny = in.ny; ff.nz = in.nz; ff.ntr = nt;
-        ff.nghost = in.nghost; ff.nxp = in.nxp; ff.nyp = in.nyp;
-        ff.wall_w = in.walls[0]; ff.wall_e = in.walls[1]; ff.wall_s = in.walls[2]; ff.wall_n = in.walls[3];
-        ff.dt = in.dt; ff.khtr = in.khtr; ff.khtr_u = in.khtr_u; ff.khtr_v = in.khtr_v;
-        ff.dy_cu = in.dy_cu; ff.dx_cv = in.dx_cv; ff.idxCu = in.idxCu; ff.idyCv = in.idyCv;
-        ff.u = in.u; ff.v = in.v; ff.ti = rc.ti; ff.ppm = rc.ppm; ff.Fu = Fu; ff.Fv = Fv;
         redi::CellGatherArgsT<P> cg{};
         cg.nx = in.nx; cg.ny = in.ny; cg.nz = in.nz; cg.ntr = nt;
         cg.nghost = in.nghost; cg.nxp = in.nxp; cg.nyp = in.nyp;
         cg.wall_w = in.walls[0]; cg.wall_e = in.walls[1]; cg.wall_s = in.walls[2]; cg.wall_n = in.walls[3];
-        cg.areaT = in.areaT; cg.u = in.u; cg.v = in.v; cg.Fu = Fu; cg.Fv = Fv; cg.err = ws.err();
+        cg.areaT = in.areaT; cg.u = in.u; cg.v = in.v; cg.Fu = ff.Fu; cg.Fv = ff.Fv; cg.err = ws.err();
         for (int n = 0; n < nt; ++n) {
             rc.htr[n] = htr_in ? htr_in[t0 + n] : htr[t0 + n];
             cg.htr[n] = htr[t0 + n];
             cg.htr_in[n] = htr_in ? htr_in[t0 + n] : htr[t0 + n];
         }
-        e = redi::launch_phase_b<P>(rc, ff, cg, st, band, t0 == 0 ? recon_from : 0);
+        e = redi::launch_phase_b<P>(rc, ff, cg, st, band, t0 == 0 ? recon_from : 0, t0 == 0 ? flux_from : 0);
         if (e != cudaSuccess) return cuda_fail(e, "phase B launch");
     }
     return REDI_B200_OK;
@@ -725,44 +745,51 @@ static int check_apply(const redi_b200_grid* grid, const redi_b200_metrics* metr
     return REDI_B200_OK;
 }
 
-// Phase B of a step whose arguments passed check_apply: the per-face KhTr
-// into the slots, then the fluxes of every tracer (recon_from: tracers of the
-// first batch already reconstructed).
-static int run_apply(const redi_b200_grid* grid, const redi_b200_metrics* metrics, redi_b200* s,
-                     const redi_b200_state* ms, double dt, const double* khtr_u_ext, const double* khtr_v_ext,
-                     const int walls[4], cudaStream_t st, int recon_from) {
-    const int nx = grid->nx_total, ny = grid->ny_total, nz = ms->nz_ml;
-    const bool use_ext = khtr_u_ext && khtr_v_ext;
-    const size_t nu = (size_t)(nx + 1) * ny, nv = (size_t)nx * (ny + 1);
-    // Resolve the per-face KhTr into the slots (:981-987).
+// The per-face KhTr into the slots (ocean_redi.F90:981-987).
+static int resolve_khtr(redi_b200* s, const double* khtr_u_ext, const double* khtr_v_ext, cudaStream_t st) {
+    const size_t nu = (size_t)(s->nx_total + 1) * s->ny_total, nv = (size_t)s->nx_total * (s->ny_total + 1);
     cudaError_t e;
-    if (use_ext) {
+    if (khtr_u_ext && khtr_v_ext) {
         e = cudaMemcpyAsync(s->khtr_u, khtr_u_ext, nu * 8, cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(s->khtr_v, khtr_v_ext, nv * 8, cudaMemcpyDeviceToDevice, st);
     } else {
         e = fill(s->khtr_u, nu, s->khtr, st);
         if (e == cudaSuccess) e = fill(s->khtr_v, nv, s->khtr, st);
     }
-    if (e != cudaSuccess) return cuda_fail(e, "redi_b200_apply_flux: khtr resolve");
-    auto fill_in = [&](auto& in) {
-        in.nx = nx; in.ny = ny; in.nz = nz; in.nghost = grid->nghost; in.nxp = grid->nx_phys; in.nyp = grid->ny_phys;
-        for (int w = 0; w < 4; ++w) in.walls[w] = walls[w];
-        in.dt = dt; in.khtr = s->khtr; in.khtr_u = s->khtr_u; in.khtr_v = s->khtr_v;
-        in.dy_cu = metrics->dy_cu; in.dx_cv = metrics->dx_cv; in.idxCu = metrics->idxCu; in.idyCv = metrics->idyCv;
-        in.areaT = metrics->areaT; in.h = ms->h_layer;
-    };
-    if (s->precision == REDI_B200_MIXED) {
-        PhaseBInputs<redi::MixedPrec> in{};
-        fill_in(in);
-        in.u = s->in_u<redi::MixedPrec>();
-        in.v = s->in_v<redi::MixedPrec>();
-        return run_phase_b<redi::MixedPrec>(in, ms->ntracers, ms->hTr, s->ws, st, nullptr, redi::Band{}, recon_from);
-    }
-    PhaseBInputs<redi::PlainPrec> in{};
-    fill_in(in);
-    in.u = s->in_u<redi::PlainPrec>();
-    in.v = s->in_v<redi::PlainPrec>();
-    return run_phase_b<redi::PlainPrec>(in, ms->ntracers, ms->hTr, s->ws, st, nullptr, redi::Band{}, recon_from);
+    return e == cudaSuccess ? REDI_B200_OK : cuda_fail(e, "redi_b200_apply_flux: khtr resolve");
+}
+
+}  // extern "C"
+
+// Phase B's inputs of a step whose arguments passed check_apply.
+template <class P>
+static PhaseBInputs<P> phase_b_inputs(const redi_b200_grid* grid, const redi_b200_metrics* metrics, redi_b200* s,
+                                      const redi_b200_state* ms, double dt, const int walls[4]) {
+    PhaseBInputs<P> in{};
+    in.nx = grid->nx_total; in.ny = grid->ny_total; in.nz = ms->nz_ml;
+    in.nghost = grid->nghost; in.nxp = grid->nx_phys; in.nyp = grid->ny_phys;
+    for (int w = 0; w < 4; ++w) in.walls[w] = walls[w];
+    in.dt = dt; in.khtr = s->khtr; in.khtr_u = s->khtr_u; in.khtr_v = s->khtr_v;
+    in.dy_cu = metrics->dy_cu; in.dx_cv = metrics->dx_cv; in.idxCu = metrics->idxCu; in.idyCv = metrics->idyCv;
+    in.areaT = metrics->areaT; in.h = ms->h_layer;
+    in.u = s->in_u<P>();
+    in.v = s->in_v<P>();
+    return in;
+}
+extern "C" {
+
+// Phase B of a step whose arguments passed check_apply: the per-face KhTr
+// into the slots, then the fluxes of every tracer.
+static int run_apply(const redi_b200_grid* grid, const redi_b200_metrics* metrics, redi_b200* s,
+                     const redi_b200_state* ms, double dt, const double* khtr_u_ext, const double* khtr_v_ext,
+                     const int walls[4], cudaStream_t st) {
+    const int r = resolve_khtr(s, khtr_u_ext, khtr_v_ext, st);
+    if (r < 0) return r;
+    if (s->precision == REDI_B200_MIXED)
+        return run_phase_b(phase_b_inputs<redi::MixedPrec>(grid, metrics, s, ms, dt, walls), ms->ntracers, ms->hTr,
+                           s->ws, st);
+    return run_phase_b(phase_b_inputs<redi::PlainPrec>(grid, metrics, s, ms, dt, walls), ms->ntracers, ms->hTr, s->ws,
+                       st);
 }
 
 int redi_b200_apply_flux(const redi_b200_grid* grid, const redi_b200_metrics* metrics, redi_b200* s,
@@ -771,59 +798,55 @@ int redi_b200_apply_flux(const redi_b200_grid* grid, const redi_b200_metrics* me
     int walls[4];
     const int chk = check_apply(grid, metrics, s, ms, khtr_u_ext, khtr_v_ext, bc, walls);
     if (chk != REDI_B200_OK) return chk;
-    return run_apply(grid, metrics, s, ms, dt, khtr_u_ext, khtr_v_ext, walls, reinterpret_cast<cudaStream_t>(stream), 0);
+    return run_apply(grid, metrics, s, ms, dt, khtr_u_ext, khtr_v_ext, walls, reinterpret_cast<cudaStream_t>(stream));
 }
-
 
 }  // extern "C"
 
-// Phase A of a whole step whose tracers 1 and 2 are T and S (either order):
-// the column state and the reconstruction of T and S in one pass, then the
-// sweep. Phase B's buffers come first in the scratch (as run_phase_b lays them
-// out for ntr tracers) and Phase A's behind them, so both live until the
-// fluxes are done; run_phase_b with recon_from = 2 follows.
+// A whole step whose tracers 1 and 2 are T and S (either order): the column
+// state and the reconstruction of T and S in one pass, the sweep with their
+// fluxes, then the rest of Phase B. Nothing can change the tracers in between.
+// Phase B's buffers come first in the scratch (as run_phase_b lays them out)
+// and Phase A's behind them, so both live until the fluxes are done. `st`
+// already carries the resolved KhTr.
 template <class P>
-static int run_fused_phase_a(int nx, int ny, int nz, int ntr, const redi::EosParams& eos, const double* h,
-                             const double* tr0, const double* tr1, int ts_swap, const double* wet_u,
-                             const double* wet_v, const redi::FaceOutT<P>& u, const redi::FaceOutT<P>& v,
-                             Scratch& ws, cudaStream_t st) {
-    const int batch = ntr < redi::kMaxTracers ? ntr : redi::kMaxTracers;
-    const size_t recon = redi::recon_bytes<P>(nx, ny, nz, batch);
-    const size_t flux = redi::flux_bytes<P>(nx, ny, nz, redi::flux_slots(batch, redi::cell_tuning()));
-    const size_t b_end = (recon + flux + 255) & ~size_t(255);
+static int run_step(const PhaseBInputs<P>& in, const redi::EosParams& eos, int ntr, double* const* htr, int ts_swap,
+                    const double* wet_u, const double* wet_v, const redi::FaceOutT<P>& u, const redi::FaceOutT<P>& v,
+                    Scratch& ws, cudaStream_t st) {
+    const int nx = in.nx, ny = in.ny, nz = in.nz;
+    const PhaseBBuffers<P> buf(nx, ny, nz, ntr);
+    const size_t b_end = (buf.recon + buf.flux + 255) & ~size_t(255);
     cudaError_t e = ws.reserve(b_end + redi::phase_a_scratch(nx, ny, nz));
     if (e != cudaSuccess) return cuda_fail(e, "scratch allocation (whole step)");
+    const redi::StepForm form = redi::step_form(buf.batch, redi::cell_tuning(),
+                                                redi::fold_shape<P>(nz, buf.batch).nt > 0, eos.variant);
+    const bool flux = form != redi::StepForm::kSeparate;
     char* base = static_cast<char*>(ws.data());
     const size_t nifc = (size_t)nx * ny * (nz + 1);
+    const redi::FaceFluxArgsT<P> ff = flux_args(in, buf, buf.batch, ws);
     redi::ColumnStateArgs cs{};
     cs.nx = nx; cs.ny = ny; cs.nz = nz; cs.eos = eos;
-    cs.h = h; cs.th = ts_swap ? tr1 : tr0; cs.sh = ts_swap ? tr0 : tr1;
+    cs.h = in.h; cs.th = htr[ts_swap ? 1 : 0]; cs.sh = htr[ts_swap ? 0 : 1];
     cs.ifc = reinterpret_cast<redi::IfcState*>(base + b_end);
     cs.pint = reinterpret_cast<double*>(cs.ifc + nifc);
     cs.wet_u = wet_u; cs.wet_v = wet_v;
     redi::ReconArgsT<P> rc{};
-    rc.nx = nx; rc.ny = ny; rc.nz = nz; rc.ntr = batch; rc.h = h;
-    rc.ti = reinterpret_cast<double*>(base);
-    rc.ppm = reinterpret_cast<typename P::Ppm*>(base + redi::recon_ppm_offset(nx, ny, nz, batch));
-    rc.htr[0] = tr0;
-    rc.htr[1] = tr1;
-    e = redi::launch_column_recon<P>(cs, rc, ts_swap, st);
+    rc.nx = nx; rc.ny = ny; rc.nz = nz; rc.ntr = buf.batch; rc.h = in.h;
+    rc.ti = const_cast<double*>(ff.ti);
+    rc.ppm = const_cast<typename P::Ppm*>(ff.ppm);
+    rc.htr[0] = htr[0];
+    rc.htr[1] = htr[1];
+    e = redi::launch_column_recon<P>(cs, rc, ts_swap, form, st);
     redi::SweepArgsT<P> sw{};
     sw.nx = nx; sw.ny = ny; sw.nz = nz; sw.rho0 = eos.rho0;
     sw.wet_u = wet_u; sw.wet_v = wet_v; sw.ifc = cs.ifc; sw.pint = cs.pint;
     sw.u = u; sw.v = v;
-    if (e == cudaSuccess) e = redi::launch_sweep<P>(sw, st);
+    sw.sv_t = eos.alpha_T / (eos.rho0 * eos.rho0);  // ocean_eos.F90:511-512
+    sw.sv_s = -eos.beta_S / (eos.rho0 * eos.rho0);
+    if (e == cudaSuccess)
+        e = flux ? redi::launch_sweep_flux<P>(sw, ff, ts_swap, form, st) : redi::launch_sweep<P>(sw, st);
     if (e != cudaSuccess) return cuda_fail(e, "phase A launch (whole step)");
-    return REDI_B200_OK;
-}
-
-template <class P>
-static int run_step_phase_a(const redi_b200_grid* grid, const redi_b200_metrics* metrics, const redi_b200_eos* eos,
-                            redi_b200* s, const redi_b200_state* ms, int ts_swap, cudaStream_t st) {
-    const redi::EosParams e{eos->variant, eos->rho0, eos->T_ref, eos->S_ref, eos->alpha_T, eos->beta_S};
-    return run_fused_phase_a<P>(grid->nx_total, grid->ny_total, ms->nz_ml, ms->ntracers, e, ms->h_layer, ms->hTr[0],
-                                ms->hTr[1], ts_swap, metrics->wet_u, metrics->wet_v, s->out_u<P>(), s->out_v<P>(),
-                                s->ws, st);
+    return run_phase_b<P>(in, ntr, htr, ws, st, nullptr, redi::Band{}, 2, flux ? 2 : 0);
 }
 
 extern "C" {
@@ -845,17 +868,22 @@ int redi_b200_step(const redi_b200_grid* grid, const redi_b200_metrics* metrics,
             if (r < 0) return r;
         }
         if (cb == REDI_B200_OK) {
-            const int r = run_apply(grid, metrics, s, ms, dt, khtr_u_ext, khtr_v_ext, walls, st, 0);
+            const int r = run_apply(grid, metrics, s, ms, dt, khtr_u_ext, khtr_v_ext, walls, st);
             if (r < 0) return r;
         }
         return (ca == REDI_B200_OK || cb == REDI_B200_OK) ? REDI_B200_OK : REDI_B200_SKIPPED;
     }
     const int ts_swap = iT == 2 ? 1 : 0;
-    const int ra = s->precision == REDI_B200_MIXED
-                       ? run_step_phase_a<redi::MixedPrec>(grid, metrics, eos, s, ms, ts_swap, st)
-                       : run_step_phase_a<redi::PlainPrec>(grid, metrics, eos, s, ms, ts_swap, st);
-    if (ra < 0) return ra;
-    return run_apply(grid, metrics, s, ms, dt, khtr_u_ext, khtr_v_ext, walls, st, 2);
+    const redi::EosParams e{eos->variant, eos->rho0, eos->T_ref, eos->S_ref, eos->alpha_T, eos->beta_S};
+    const int r = resolve_khtr(s, khtr_u_ext, khtr_v_ext, st);
+    if (r < 0) return r;
+    if (s->precision == REDI_B200_MIXED)
+        return run_step(phase_b_inputs<redi::MixedPrec>(grid, metrics, s, ms, dt, walls), e, ms->ntracers, ms->hTr,
+                        ts_swap, metrics->wet_u, metrics->wet_v, s->out_u<redi::MixedPrec>(),
+                        s->out_v<redi::MixedPrec>(), s->ws, st);
+    return run_step(phase_b_inputs<redi::PlainPrec>(grid, metrics, s, ms, dt, walls), e, ms->ntracers, ms->hTr,
+                    ts_swap, metrics->wet_u, metrics->wet_v, s->out_u<redi::PlainPrec>(),
+                    s->out_v<redi::PlainPrec>(), s->ws, st);
 }
 
 }  // extern "C"
@@ -1058,9 +1086,6 @@ static void compat_launch(const char* name, const int* nx_, const int* ny_, cons
     cudaStream_t st = 0;  // the reference launches on the legacy default stream
     redi::EosParams e{1, *rho0_, *T_ref_, *S_ref_, *alpha_T_, *beta_S_};  // the launcher's LINEAR EOS
     redi::FaceOut u{uPoL, uPoR, uKoL, uKoR, uhEff, udry}, v{vPoL, vPoR, vKoL, vKoR, vhEff, vdry};
-    // both phases in this call: the column state and the T/S reconstruction in one pass
-    int rc = run_fused_phase_a<redi::PlainPrec>(nx, ny, nz, 2, e, h_layer, t_htr, s_htr, 0, wet_u, wet_v, u, v, ws, st);
-    if (rc < 0) { report(rc, g_last_error); return; }
     cudaMemcpyAsync(khtr_u, khtr_u_ext, nu * 8, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(khtr_v, khtr_v_ext, nv * 8, cudaMemcpyDeviceToDevice, st);
     PhaseBInputs<redi::PlainPrec> in{};
@@ -1071,7 +1096,7 @@ static void compat_launch(const char* name, const int* nx_, const int* ny_, cons
     in.u = redi::FaceIn{uPoL, uPoR, uKoL, uKoR, uhEff, udry};
     in.v = redi::FaceIn{vPoL, vPoR, vKoL, vKoR, vhEff, vdry};
     double* trs[2] = {t_htr, s_htr};
-    rc = run_phase_b<redi::PlainPrec>(in, 2, trs, ws, st, nullptr, redi::Band{}, 2);
+    const int rc = run_step(in, e, 2, trs, 0, wet_u, wet_v, u, v, ws, st);
     if (rc < 0) { report(rc, g_last_error); return; }
     cudaDeviceSynchronize();
 }

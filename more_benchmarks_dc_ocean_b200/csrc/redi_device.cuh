@@ -15,6 +15,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 namespace redi {
@@ -26,6 +27,13 @@ struct LdNC {
     template <class T>
     __device__ static __forceinline__ T ld(const T* p) { return __ldg(p); }
 };
+// A 32-byte record (32-byte aligned) in one load: a warp's request then touches
+// each 128-byte line once instead of twice.
+__device__ __forceinline__ double4 ld256_nc(const void* p) {
+    double4 r;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    return r;
+}
 struct LdCG {
     template <class T>
     __device__ static __forceinline__ T ld(const T* p) { return __ldcg(p); }
@@ -55,15 +63,19 @@ struct PlmGeom {
     bool ok;            // (h(k+1)+h(k))*(h(k-1)+h(k)) > 0
 };
 
-__device__ __forceinline__ PlmGeom plm_geom(double hkm1, double hk, double hkp1) {
+// The reciprocal of the sum of two neighbouring layers, as the slope below the
+// pair, the slope above it and the edge between them all use it (a zero stays).
+__device__ __forceinline__ double pair_inverse(double ha, double hb) {
+    const double s = ha + hb;
+    return s != 0.0 ? 1.0 / s : s;
+}
+
+// hm, hp: pair_inverse of (hkm1, hk) and (hk, hkp1).
+__device__ __forceinline__ PlmGeom plm_geom(double hkm1, double hk, double hkp1, double hm, double hp) {
     PlmGeom g;
     g.ok = (hkp1 + hk) * (hkm1 + hk) > 0.0;
     double h_sum = (hkm1 + hkp1) + hk;
     if (h_sum != 0.0) h_sum = 1.0 / h_sum;
-    double hm = hkm1 + hk;
-    if (hm != 0.0) hm = 1.0 / hm;
-    double hp = hkp1 + hk;
-    if (hp != 0.0) hp = 1.0 / hp;
     g.g0 = hk * h_sum;
     g.g1 = (2.0 * hkm1 + hk) * hp;
     g.g2 = (2.0 * hkp1 + hk) * hm;
@@ -105,16 +117,15 @@ struct EdgeGeom {
     bool lt;          // hk < hkp1 selects the interpolation anchor
 };
 
-__device__ __forceinline__ EdgeGeom edge_geom(double hkm1, double hk, double hkp1, double hkp2, double hn) {
+// r: pair_inverse of (hk, hkp1).
+__device__ __forceinline__ EdgeGeom edge_geom(double hkm1, double hk, double hkp1, double hkp2, double hn, double r) {
     EdgeGeom g;
-    double r = hk + hkp1;
-    g.degenerate = r <= 0.0;
+    g.degenerate = hk + hkp1 <= 0.0;
     g.lt = hk < hkp1;
     if (g.degenerate) {
         g.w = g.f1 = g.f2 = g.f3 = g.f4 = 0.0;
         return g;
     }
-    r = 1.0 / r;
     g.w = g.lt ? hk * r : hkp1 * r;
     double r_2hk_hkp1 = 1.0 / ((2.0 * hk + hkp1) + hn);
     double r_hk_2hkp1 = 1.0 / ((hk + 2.0 * hkp1) + hn);
@@ -191,10 +202,15 @@ __device__ __forceinline__ PpmLayer make_ppm_layer(double alk, double ark, doubl
 
 template <class LD>
 __device__ __forceinline__ PpmLayer load_ppm(const PpmLayer* p) {
-    const double2* q = reinterpret_cast<const double2*>(p);
-    double2 a = LD::ld(q), b = LD::ld(q + 1);
     PpmLayer r;
-    r.aL = a.x; r.dA = a.y; r.a6o3 = b.x; r.B = b.y;
+    if constexpr (std::is_same<LD, LdNC>::value) {
+        const double4 a = ld256_nc(p);
+        r.aL = a.x; r.dA = a.y; r.a6o3 = a.z; r.B = a.w;
+    } else {
+        const double2* q = reinterpret_cast<const double2*>(p);
+        double2 a = LD::ld(q), b = LD::ld(q + 1);
+        r.aL = a.x; r.dA = a.y; r.a6o3 = b.x; r.B = b.y;
+    }
     return r;
 }
 
@@ -219,11 +235,14 @@ __device__ __forceinline__ void ppm_limit(double& alk, double& ark, double tlk) 
     }
 }
 
-// redi_sublayer_dT's down-gradient guard (ocean_redi.F90:919-924).
+// redi_sublayer_dT's down-gradient guard (ocean_redi.F90:919-924): the top and
+// bottom differences must agree in sign, and their mean with the layer's
+// (a zero agrees with nothing). Once top and bottom agree their mean is not
+// zero and has their sign, so the three signs are compared directly.
 __device__ __forceinline__ double guarded_dT(double dT_top, double dT_bot, double dT_layer) {
-    double dT_ave = 0.5 * (dT_top + dT_bot);
-    if (signs_not_agree(dT_top, dT_bot) || signs_not_agree(dT_ave, dT_layer)) return 0.0;
-    return dT_layer;
+    const int s = __double2hiint(dT_top);
+    const bool same = ((s ^ __double2hiint(dT_bot)) | (s ^ __double2hiint(dT_layer))) >= 0;
+    return same && dT_top != 0.0 && dT_bot != 0.0 && dT_layer != 0.0 ? dT_layer : 0.0;
 }
 
 }  // namespace redi

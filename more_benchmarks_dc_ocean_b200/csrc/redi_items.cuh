@@ -70,6 +70,8 @@ __device__ __forceinline__ void stream_edges(int nk, Fetch fetch, Emit emit) {
         sB[n] = 0.0;
     }
     emit(1, e, sB, hC);
+    // 1/(h(t-1) + h(t)): one division a layer for the two slopes and the edge that share it
+    double rBC = nk >= 2 ? pair_inverse(hC, hD) : 0.0, rCD = 0.0;
 
     for (int t = 2; t <= nk; ++t) {
         // shift the window down one layer: (t-1) <- t, t <- t+1
@@ -93,7 +95,8 @@ __device__ __forceinline__ void stream_edges(int nk, Fetch fetch, Emit emit) {
         }
         // diff(t): PLM slope for 2 <= t <= nk-1, PCM (0) at t = nk.
         if (t <= nk - 1) {
-            const PlmGeom pg = plm_geom(hB, hC, hD);
+            rCD = pair_inverse(hC, hD);
+            const PlmGeom pg = plm_geom(hB, hC, hD, rBC, rCD);
 #pragma unroll
             for (int n = 0; n < NS; ++n) dC[n] = plm_slope(pg, sB[n], sC[n], sD[n]);
         } else {
@@ -102,7 +105,8 @@ __device__ __forceinline__ void stream_edges(int nk, Fetch fetch, Emit emit) {
         }
         const double hkm1 = (t >= 3) ? hA : hB;   // h(max(1, t-2))
         const double hkp2 = (t + 1 <= nk) ? hD : hC;  // h(min(nk, t+1))
-        const EdgeGeom eg = edge_geom(hkm1, hB, hC, hkp2, kHNeglect);
+        const EdgeGeom eg = edge_geom(hkm1, hB, hC, hkp2, kHNeglect, rBC);
+        rBC = rCD;
 #pragma unroll
         for (int n = 0; n < NS; ++n) e[n] = ppm_edge(eg, sB[n], sC[n], dB[n], dC[n]);
         emit(t, e, sB, hC);
@@ -523,38 +527,69 @@ __device__ __forceinline__ void sweep_item(const SweepArgsT<P>& a, int dir, int 
 // non-zero value).
 // ---------------------------------------------------------------------------
 constexpr int kSweepWinThreads = 128;  // block size of the shared-memory-window sweep
+//
+// LIN: the packed column state of a linear equation of state: its derivatives
+// are one value per interface, m = -(rho * rho), times two constants of the
+// run, so an interface is {T, S, m, P}: 32 bytes in one sector instead of 40 in
+// two, two copies and no separate pressure read. The products m * sv_t and
+// m * sv_s are the column state's own.
+template <int NR, bool LIN = false>
+struct SweepWin;
 template <int NR>
-struct SweepWin {
+struct SweepWin<NR, false> {
     double2 ts[NR][2][kSweepWinThreads];  // (T, S)
     double2 dd[NR][2][kSweepWinThreads];  // (dR/dT, dR/dS)
     double p[NR][2][kSweepWinThreads];    // pressure
 };
-
 template <int NR>
-__device__ __forceinline__ void sw_fetch(SweepWin<NR>& r, int side, int q, const IfcState* X, const double* P, int nk,
-                                         size_t ld) {
-    const int slot = q % NR, qi = min(q, nk), tid = threadIdx.x;
-    const double2* src = reinterpret_cast<const double2*>(X + (size_t)qi * ld);
-    cp_async16(&r.ts[slot][side][tid], src);
-    cp_async16(&r.dd[slot][side][tid], src + 1);
-    cp_async8(&r.p[slot][side][tid], P + (size_t)qi * ld);
+struct SweepWin<NR, true> {
+    double2 ts[NR][2][kSweepWinThreads];  // (T, S)
+    double2 mp[NR][2][kSweepWinThreads];  // (m, pressure)
+};
+
+// Byte offset in the ring of (T, S) of interface q; `t` is the thread's (and
+// side's) offset in a slot. The second pair sits kDd behind it, the pressure
+// kP + half of it (packed: in the second pair). Unsigned arithmetic: a slot is
+// one mask for NR = 4.
+template <int NR>
+struct RingAt {
+    static constexpr unsigned kSide = kSweepWinThreads * sizeof(double2), kSlot = 2 * kSide;
+    static constexpr unsigned kDd = NR * kSlot, kP = 2 * kDd;
+    __device__ static __forceinline__ unsigned at(unsigned t, int q) { return t + ((unsigned)q % NR) * kSlot; }
+};
+
+// The ring slot of interface q of the column at index `idx` = min(q, nk) * ld + column.
+template <int NR, bool LIN>
+__device__ __forceinline__ void sw_fetch(SweepWin<NR, LIN>& r, unsigned o, unsigned idx, const IfcState* X,
+                                         const double* P) {
+    char* base = reinterpret_cast<char*>(&r);
+    const double2* src = reinterpret_cast<const double2*>(X + idx);
+    cp_async16(base + o, src);
+    cp_async16(base + RingAt<NR>::kDd + o, src + 1);
+    if constexpr (!LIN) cp_async8(base + RingAt<NR>::kP + (o >> 1), P + idx);
 }
 
-template <int NR>
-__device__ __forceinline__ IfcState sw_ifc(const SweepWin<NR>& r, int side, int q) {
-    const int slot = q % NR, tid = threadIdx.x;
-    const double2 a = r.ts[slot][side][tid], b = r.dd[slot][side][tid];
+template <int NR, bool LIN>
+__device__ __forceinline__ double2 sw_ts(const SweepWin<NR, LIN>& r, unsigned o) {
+    return *reinterpret_cast<const double2*>(reinterpret_cast<const char*>(&r) + o);
+}
+
+template <int NR, bool LIN>
+__device__ __forceinline__ IfcState sw_ifc(const SweepWin<NR, LIN>& r, unsigned o, double sv_t, double sv_s) {
+    const double2 a = sw_ts(r, o), b = sw_ts(r, o + RingAt<NR>::kDd);
     IfcState s;
     s.T = a.x;
     s.S = a.y;
-    s.dRdT = b.x;
-    s.dRdS = b.y;
+    s.dRdT = LIN ? b.x * sv_t : b.x;
+    s.dRdS = LIN ? b.x * sv_s : b.y;
     return s;
 }
 
-template <int NR>
-__device__ __forceinline__ double sw_p(const SweepWin<NR>& r, int side, int q) {
-    return r.p[q % NR][side][threadIdx.x];
+template <int NR, bool LIN>
+__device__ __forceinline__ double sw_p(const SweepWin<NR, LIN>& r, unsigned o) {
+    const char* base = reinterpret_cast<const char*>(&r);
+    return *reinterpret_cast<const double*>(LIN ? base + RingAt<NR>::kDd + sizeof(double) + o
+                                                : base + RingAt<NR>::kP + (o >> 1));
 }
 
 // Ordered compaction across a block of NT threads: the threads whose `keep`
@@ -617,164 +652,177 @@ __device__ __forceinline__ bool sweep_face_dry(const SweepArgsT<P>& a, int dir, 
     return false;
 }
 
+// What else a sweep does with each surface: `begin()` as a step begins and `surface(ks, so, pol, por, kol,
+// kor, he)` once surface ks (1-based, at offset so of its slots) is placed, with
+// the effective thickness he of the sublayer above it (ks > 1). Interfaces ko-1
+// and ko (0-based) of either side are then in the ring.
+struct NoSink {
+    __device__ __forceinline__ void begin() {}
+    template <class He>
+    __device__ __forceinline__ void surface(int, unsigned, double, double, int, int, He) {}
+};
+
 // r: this block's ring (dynamic shared memory, blocks of kSweepThreads).
 // WET_ONLY: the caller has run sweep_face_dry and t is a wet face.
-template <class P, class LD, int NR, bool WET_ONLY = false>
-__device__ __forceinline__ void sweep_item_win(const SweepArgsT<P>& a, int dir, int t, SweepWin<NR>& r) {
+//
+// The step is bound by the instructions it issues, so: one direction flag
+// (the two of the reference are each other's complement from the first step
+// on), 32-bit slot and scratch indices (a domain has fewer than 2^31 of
+// either), the clamp of the interpolated position reduced to the two
+// comparisons that can matter (a step reaches the division only with
+// dRhoTop < dRhoBot, both ordered, so the quotient's divisor is positive; an
+// infinite pair gives NaN, which clamps to 0 as fmax and fmin do), and the
+// monotonic test without an integer conversion (a side's layer is its
+// pointer's or the one above, so it moves by -1, 0 or 1, and a rounded sum has
+// the sign of the exact one).
+template <class P, class LD, int NR, bool WET_ONLY = false, bool LIN = false, class Sink = NoSink>
+__device__ __forceinline__ void sweep_item_win(const SweepArgsT<P>& a, int dir, int t, SweepWin<NR, LIN>& r,
+                                               Sink sink = Sink{}) {
     static_assert(NR >= 3 && NR <= 5, "ring of 3 (none in flight), 4 (one) or 5 (two)");
-    const int nx = a.nx, ny = a.ny, nz = a.nz, ns = 2 * nz + 2;
-    const size_t ld = (size_t)nx * ny;
-    int colL, colR, fo;
-    size_t fstride;
+    using At = RingAt<NR>;
+    const int nx = a.nx, ny = a.ny, nk = a.nz, ns = 2 * nk + 2;
+    const unsigned ld = (unsigned)nx * ny;
+    unsigned colL, colR, fo, fstride;
     if (dir == 0) {
         if (t >= (nx - 1) * ny) return;
         const int j = t / (nx - 1), fi = 1 + t % (nx - 1);
         colL = (fi - 1) + nx * j;
         colR = fi + nx * j;
         fo = fi + (nx + 1) * j;
-        fstride = (size_t)(nx + 1) * ny;
+        fstride = (unsigned)(nx + 1) * ny;
     } else {
         if (t >= nx * (ny - 1)) return;
         const int fj = 1 + t / nx, i = t % nx;
         colL = i + nx * (fj - 1);
         colR = i + nx * fj;
         fo = i + nx * fj;
-        fstride = (size_t)nx * (ny + 1);
+        fstride = (unsigned)nx * (ny + 1);
     }
     using Po = typename P::Po;
     using Ko = typename P::Ko;
     using He = typename P::He;
-    const FaceOutT<P> o = dir == 0 ? a.u : a.v;
-    Po* __restrict__ PoL = o.PoL + fo;
-    Po* __restrict__ PoR = o.PoR + fo;
-    Ko* __restrict__ KoL = o.KoL + fo;
-    Ko* __restrict__ KoR = o.KoR + fo;
-    He* __restrict__ hEff = o.hEff + fo;
+    const FaceOutT<P>& o = dir == 0 ? a.u : a.v;
+    Po* __restrict__ const PoL = o.PoL;
+    Po* __restrict__ const PoR = o.PoR;
+    Ko* __restrict__ const KoL = o.KoL;
+    Ko* __restrict__ const KoR = o.KoR;
+    He* __restrict__ const hEff = o.hEff;
     if constexpr (!WET_ONLY) {
         if (!sweep_face_dry<P, LD>(a, dir, t)) return;
     }
 
-    const IfcState* XL = a.ifc + colL;
-    const IfcState* XR = a.ifc + colR;
-    const double* PL = a.pint + colL;
-    const double* PR = a.pint + colR;
     const double pa_to_h = 1.0 / (kGravity * a.rho0);
-    const int nk = nz;
+    const double svt = a.sv_t, svs = a.sv_s;
     constexpr int kAhead = NR - 3;  // interfaces in flight beyond the window
+    const unsigned tL = threadIdx.x * (unsigned)sizeof(double2), tR = tL + At::kSide;
 
 #pragma unroll
     for (int q = 0; q < 3 + kAhead; ++q) {
-        sw_fetch(r, 0, q, XL, PL, nk, ld);
-        sw_fetch(r, 1, q, XR, PR, nk, ld);
+        const unsigned qi = (unsigned)min(q, nk) * ld;
+        sw_fetch(r, At::at(tL, q), qi + colL, a.ifc, a.pint);
+        sw_fetch(r, At::at(tR, q), qi + colR, a.ifc, a.pint);
     }
     cp_async_commit();
     cp_async_wait<0>();
 
-    int kL = 1, kR = 1;
+    int kl = 1, kr = 1;
     double lastP_left = 0.0, lastP_right = 0.0;
     int lastK_left = 1, lastK_right = 1;
-    bool reached_bottom = false, search_left = false, search_right = false;
+    bool reached_bottom = false, left = false;
     double absL_prev = 0.0, absR_prev = 0.0;
+    unsigned so = fo;  // this surface's slot
 
-    for (int ks = 1; ks <= ns; ++ks) {
+    for (int ks = 1; ks <= ns; ++ks, so += fstride) {
+        sink.begin();
         if constexpr (kAhead == 0) cp_async_wait<0>();
-        const int kl = kL, kr = kR;
-        const IfcState oL = sw_ifc(r, 0, kl - 1), oR = sw_ifc(r, 1, kr - 1);
-        const double dRho = secant_drho(oR, oL);
-        if (!reached_bottom) {
-            if (dRho < 0.0) {
-                search_left = true;
-                search_right = false;
-            } else if (dRho > 0.0) {
-                search_right = true;
-                search_left = false;
-            } else if (kl + kr == 2) {
-                search_left = true;
-                search_right = false;
-            } else {
-                search_left = !search_left;
-                search_right = !search_right;
-            }
-        }
-        const bool L = search_left;
-        const int sS = L ? 0 : 1, sA = L ? 1 : 0;
+        const unsigned ownL = At::at(tL, kl - 1), ownR = At::at(tR, kr - 1);
+        const double dRho = secant_drho(sw_ifc(r, ownR, svt, svs), sw_ifc(r, ownL, svt, svs));
+        if (!reached_bottom) left = dRho < 0.0 || (!(dRho > 0.0) && (kl + kr == 2 || !left));
+        const bool L = left;
+        const unsigned tS = L ? tL : tR, tA = L ? tR : tL;
+        const unsigned ownA = L ? ownR : ownL;
         const int Sk = L ? kl : kr, ka = L ? kr : kl;
-        const int w0 = Sk > 2 ? Sk - 2 : 0;  // the searched column's km1, 0-based
-        const IfcState Sa = sw_ifc(r, sS, w0);
-        const IfcState anc = sw_ifc(r, sA, ka - 1);
-        const double dRhoTop = secant_drho(Sa, anc);
-        const double dRhoBot = Sk >= 2 ? (L ? -dRho : dRho) : secant_drho(sw_ifc(r, sS, w0 + 1), anc);
-        const double Spa = sw_p(r, sS, w0), Spb = sw_p(r, sS, w0 + 1);
-        const int km1 = w0 + 1;
-        double po_s;
-        const bool top_zero = (L ? (dRhoTop > 0.0) : (dRhoTop >= 0.0)) || kr + kl == 2;
-        if (top_zero) po_s = 0.0;
-        else if (dRhoTop >= dRhoBot) po_s = 1.0;
-        else po_s = interpolate_position(dRhoTop, Spa, dRhoBot, Spb);
-        int ko_s = km1;
-        bool carried = false;
-        if (po_s >= 1.0 && km1 < nk) {
-            ko_s = km1 + 1;
-            po_s = po_s - 1.0;
-            carried = true;
+        const int km1 = max(Sk - 1, 1);  // the reference's km1 (1-based): interfaces km1-1 and km1 (0-based)
+        const unsigned oSa = At::at(tS, km1 - 1), oSb = At::at(tS, km1);
+        const IfcState anc = sw_ifc(r, ownA, svt, svs);
+        const double dRhoTop = secant_drho(sw_ifc(r, oSa, svt, svs), anc);
+        const double dRhoBot = Sk >= 2 ? (L ? -dRho : dRho) : secant_drho(sw_ifc(r, oSb, svt, svs), anc);
+        const double Spa = sw_p(r, oSa), Spb = sw_p(r, oSb);
+        // redi_interpolate_position (ocean_redi.F90:260-285) and its callers' tests
+        const bool zero = (L ? dRhoTop > 0.0 : dRhoTop >= 0.0) || kr + kl == 2;
+        const bool one = dRhoTop >= dRhoBot;
+        double po_s = zero ? 0.0 : one ? 1.0 : 0.5;
+        if (!zero && !one && Spb > Spa && dRhoTop < dRhoBot) {
+            const double x = -dRhoTop / (dRhoBot - dRhoTop);
+            po_s = x > 0.0 ? x : 0.0;
+            po_s = po_s < 1.0 ? po_s : 1.0;
         }
+        // a position at the layer's bottom is carried into the layer below
+        const double Spc = sw_p(r, At::at(tS, km1 + 1));
+        const bool carried = po_s >= 1.0 && km1 < nk;
+        int ko_s = carried ? km1 + 1 : km1;
+        po_s = carried ? po_s - 1.0 : po_s;
+        const double p0 = carried ? Spb : Spa, p1 = carried ? Spc : Spb;
+        double abs_s = p0 + po_s * (p1 - p0);
+        // monotonic backstop
         const int lastK_s = L ? lastK_left : lastK_right;
         const double lastP_s = L ? lastP_left : lastP_right;
-        bool backstop = false;
-        if ((double)(ko_s - lastK_s) + (po_s - lastP_s) < 0.0) {
-            po_s = lastP_s;
-            ko_s = lastK_s;
-            backstop = true;
-        }
-        double abs_s;
-        if (backstop) abs_s = L ? absL_prev : absR_prev;
-        else if (carried) abs_s = Spb + po_s * (sw_p(r, sS, w0 + 2) - Spb);
-        else abs_s = Spa + po_s * (Spb - Spa);
+        const double abs_prev_s = L ? absL_prev : absR_prev;
+        const int dk = ko_s - lastK_s;
+        const bool back = po_s - lastP_s < (dk == 0 ? 0.0 : dk > 0 ? -1.0 : 1.0);
+        po_s = back ? lastP_s : po_s;
+        ko_s = back ? lastK_s : ko_s;
+        abs_s = back ? abs_prev_s : abs_s;
         double po_a, abs_a;
         int ko_a;
         if (ka <= nk) {
             po_a = 0.0;
             ko_a = ka;
-            abs_a = sw_p(r, sA, ka - 1);
+            abs_a = sw_p(r, ownA);
             // the anchor column advances: its window slides once k >= 2, and
             // the slot that left it receives the interface kAhead + 2 below
-            // the one that entered
-            if (ka >= 2) {
-                if constexpr (kAhead == 2) cp_async_wait<1>();
-                else if constexpr (kAhead == 1) cp_async_wait<0>();
-                sw_fetch(r, sA, ka + kAhead + 1, L ? XR : XL, L ? PR : PL, nk, ld);
-                cp_async_commit();
-            }
-            if (L) kR = ka + 1;
-            else kL = ka + 1;
+            // the one that entered (at k = 1 nothing slides, and the newest
+            // interface is fetched once more)
+            if constexpr (kAhead == 2) cp_async_wait<1>();
+            else if constexpr (kAhead == 1) cp_async_wait<0>();
+            const int q = ka + kAhead + 1;
+            sw_fetch(r, At::at(tA, q), (unsigned)min(q, nk) * ld + (L ? colR : colL), a.ifc, a.pint);
+            cp_async_commit();
+            kr += L ? 1 : 0;
+            kl += L ? 0 : 1;
         } else {
             po_a = 1.0;
             ko_a = nk;
-            const double Apa = sw_p(r, sA, ka - 2), Apb = sw_p(r, sA, ka - 1);
+            const double Apa = sw_p(r, At::at(tA, ka - 2)), Apb = sw_p(r, ownA);
             abs_a = Apa + po_a * (Apb - Apa);  // km1 = nk: interfaces nk, nk+1
             reached_bottom = true;
-            search_left = !L;
-            search_right = L;
+            left = !L;
         }
         const double pol = L ? po_s : po_a, por = L ? po_a : po_s;
         const int kol = L ? ko_s : ko_a, kor = L ? ko_a : ko_s;
         const double absL = L ? abs_s : abs_a, absR = L ? abs_a : abs_s;
-        lastK_left = kol;
-        lastP_left = pol;
-        lastK_right = kor;
-        lastP_right = por;
-        const size_t so = (size_t)(ks - 1) * fstride;
         PoL[so] = Po(pol);
         PoR[so] = Po(por);
         KoL[so] = Ko(kol);
         KoR[so] = Ko(kor);
+        He hv = He(0);
         if (ks > 1) {  // harmonic-mean effective thickness (:452-462), Pa -> m (:688-691)
             const double hL = absL - absL_prev;
             const double hR = absR - absR_prev;
             double he = 0.0;
-            if (hL + hR > 0.0) he = 2.0 * hL * hR / (hL + hR);
-            hEff[so - fstride] = He(he * pa_to_h);
+            if (hL + hR > 0.0) {
+                he = 2.0 * hL * hR;
+                // a zero product is its own quotient; dividing it would send the warp down the division's slow path
+                if (he != 0.0) he = he / (hL + hR);
+            }
+            hv = He(he * pa_to_h);
+            hEff[so - fstride] = hv;
         }
+        sink.surface(ks, so, pol, por, kol, kor, hv);
+        lastK_left = kol;
+        lastP_left = pol;
+        lastK_right = kor;
+        lastP_right = por;
         absL_prev = absL;
         absR_prev = absR;
     }
@@ -866,7 +914,10 @@ __device__ __forceinline__ void recon_item(const ReconArgsT<P>& a, int gid, int 
 // those of the two passes bit for bit. A column none of whose faces is wet is
 // read by neither the sweep nor the face flux, and is skipped.
 // ---------------------------------------------------------------------------
-template <class P, class LD>
+// TI: also write the interface values (the face flux inside the sweep takes
+// T and S from the column state). LIN: a linear equation of state, the column
+// state packed as the sweep's packed ring takes it (SweepWin).
+template <class P, class LD, bool TI, bool LIN>
 __device__ __forceinline__ void column_recon_item(const ColumnStateArgs& a, const ReconArgsT<P>& rc, int ts_swap,
                                                   int col) {
     const int ncol = a.nx * a.ny;
@@ -907,19 +958,23 @@ __device__ __forceinline__ void column_recon_item(const ColumnStateArgs& a, cons
         if (t >= 2) pres = pres + grho * h_layer_above;
         const double eT = e[iT], eS = e[iS];
         double rho_i, sv_t = dsv_dt, sv_s = dsv_ds;
-        if (linear)
+        if (LIN || linear)
             rho_i = eos.rho0 + eos.beta_S * (eS - eos.S_ref) - eos.alpha_T * (eT - eos.T_ref);
         else
             eos::nonlinear_point(eos.variant, eT, eS, pres, rho_i, sv_t, sv_s);
         double2* q = reinterpret_cast<double2*>(ifc + (size_t)(t - 1) * ncol);
         q[0] = make_double2(eT, eS);
-        q[1] = make_double2(-(rho_i * rho_i) * sv_t, -(rho_i * rho_i) * sv_s);
-        pint[(size_t)(t - 1) * ncol] = pres;
+        if constexpr (LIN) {
+            q[1] = make_double2(-(rho_i * rho_i), pres);
+        } else {
+            q[1] = make_double2(-(rho_i * rho_i) * sv_t, -(rho_i * rho_i) * sv_s);
+            pint[(size_t)(t - 1) * ncol] = pres;
+        }
         h_layer_above = h_t;
         // reconstruction (recon_item)
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
-            ti[n][(size_t)(t - 1) * ncol] = e[n];
+            if constexpr (TI) ti[n][(size_t)(t - 1) * ncol] = e[n];
             if (t >= 2) {
                 double alk = e_prev[n], ark = e[n];
                 const double tlk = s_above[n];
@@ -960,6 +1015,18 @@ struct FluxOps<PlainPrec> {
         return load_ppm<LD>(p);
     }
     __device__ static __forceinline__ double mean(double xL, double xR, const Raw& q) { return ppm_ave(xL, xR, q); }
+    // mean() of two tracers over the same interval: one branch, the interval's polynomial terms once
+    __device__ static __forceinline__ void mean2(double xL, double xR, const Raw (&q)[2], double (&m)[2]) {
+        const double dx = xR - xL;
+        if (dx > 0.0 && dx <= 1.0) {
+            const double xave = 0.5 * (xR + xL), xx = xR * xR + xR * xL + xL * xL;
+            m[0] = (q[0].aL + xave * q[0].B) - q[0].a6o3 * xx;
+            m[1] = (q[1].aL + xave * q[1].B) - q[1].a6o3 * xx;
+        } else {
+            m[0] = ppm_ave(xL, xR, q[0]);
+            m[1] = ppm_ave(xL, xR, q[1]);
+        }
+    }
     __device__ static __forceinline__ double flux(double dT, double he, double coef) { return dT * he * coef; }
 };
 
@@ -982,6 +1049,18 @@ struct FluxOps<MixedPrec> {
         }
         const float a6 = 3.0f * q.z;
         return q.x + q.y * xr + a6 * xr * (1.0f - xr);
+    }
+    __device__ static __forceinline__ void mean2(double xL, double xR, const Raw (&q)[2], float (&m)[2]) {
+        const double dx = xR - xL;
+        if (dx > 0.0 && dx <= 1.0) {
+            const float xl = (float)xL, xr = (float)xR;
+            const float xave = 0.5f * (xr + xl), xx = xr * xr + xr * xl + xl * xl;
+            m[0] = (q[0].x + xave * q[0].w) - q[0].z * xx;
+            m[1] = (q[1].x + xave * q[1].w) - q[1].z * xx;
+        } else {
+            m[0] = mean(xL, xR, q[0]);
+            m[1] = mean(xL, xR, q[1]);
+        }
     }
     __device__ static __forceinline__ float flux(double dT, float he, double coef) {
         return (float)dT * he * (float)coef;
@@ -1170,6 +1249,116 @@ __device__ __forceinline__ void flux_item(const FaceFluxArgsT<P>& a, int dir, in
         pr_c = pr_n;
     }
 }
+
+// ---------------------------------------------------------------------------
+// The face flux of T and S inside the sweep (a whole step in one call): the
+// sink of a face's sweep. The sublayer between surfaces ks-1 and ks is
+// evaluated as soon as the sweep has placed surface ks, with positions, layers
+// and thickness in registers and the interface values of T and S (the
+// reconstruction's own) in the sweep's ring; only the limited PPM layers are
+// read from memory, at the beginning of the step that needs them. The
+// coefficients are not read back. Values and stores are flux_item's.
+// ---------------------------------------------------------------------------
+template <class P, class LD, int NR, bool LIN>
+struct FluxSink {
+    using Ops = FluxOps<P>;
+    using Raw = typename Ops::Raw;
+    using Flux = typename P::Flux;
+    const SweepWin<NR, LIN>& r;
+    const typename P::Ppm* ppT;  // limited layers of T and of S, [layer][column]
+    const typename P::Ppm* ppS;
+    Flux* FT;               // flux of T and of S, the direction's slots
+    Flux* FS;
+    unsigned colL, colR, ncol, fstride;
+    double coef;
+    int ns;
+    bool on;  // not a wall: its fluxes are read by the gather
+    // the top surface of the next sublayer and its layers
+    double pl = 0.0, pr = 0.0;
+    double2 tl, tr;
+    int kl = 0, kr = 0;
+    Raw qL[2] = {}, qR[2] = {};
+
+    // a: a launch whose tracers 0 and 1 are T and S (S and T when ts_swap)
+    __device__ __forceinline__ FluxSink(const FaceFluxArgsT<P>& a, const SweepWin<NR, LIN>& ring, int ts_swap,
+                                        int dir, int t)
+        : r(ring), ncol((unsigned)a.nx * a.ny), ns(2 * a.nz + 2) {
+        const int nx = a.nx, ny = a.ny;
+        int fo;
+        if (dir == 0) {
+            const int j = t / (nx - 1), fi = 1 + t % (nx - 1), I = fi + 1;
+            on = !((a.wall_w && I == a.nghost + 1) || (a.wall_e && I == a.nghost + a.nxp + 1));
+            colL = (fi - 1) + nx * j;
+            colR = fi + nx * j;
+            fo = fi + (nx + 1) * j;
+            fstride = (unsigned)(nx + 1) * ny;
+        } else {
+            const int fj = 1 + t / nx, i = t % nx, J = fj + 1;
+            on = !((a.wall_s && J == a.nghost + 1) || (a.wall_n && J == a.nghost + a.nyp + 1));
+            colL = i + nx * (fj - 1);
+            colR = i + nx * fj;
+            fo = i + nx * fj;
+            fstride = (unsigned)nx * (ny + 1);
+        }
+        const double* kh = dir == 0 ? a.khtr_u : a.khtr_v;
+        const double khv = kh ? LD::ld(kh + fo) : a.khtr;
+        coef = a.dt * khv * LD::ld((dir == 0 ? a.dy_cu : a.dx_cv) + fo) * LD::ld((dir == 0 ? a.idxCu : a.idyCv) + fo);
+        Flux* const F0 = dir == 0 ? a.Fu : a.Fv;
+        Flux* const F1 = F0 + (size_t)(ns - 1) * fstride;
+        FT = ts_swap ? F1 : F0;
+        FS = ts_swap ? F0 : F1;
+        const typename P::Ppm* const p1 = a.ppm + (size_t)ncol * a.nz;
+        ppT = ts_swap ? p1 : a.ppm;
+        ppS = ts_swap ? a.ppm : p1;
+    }
+
+    __device__ __forceinline__ void layers(unsigned x, Raw (&q)[2]) const {
+        q[0] = Ops::template load<LD>(ppT + x);
+        q[1] = Ops::template load<LD>(ppS + x);
+    }
+    __device__ __forceinline__ Flux flux(double tL, double tR, double bL, double bR, typename Ops::Mean mL,
+                                         typename Ops::Mean mR, typename P::He he) const {
+        return Ops::flux(guarded_dT(tR - tL, bR - bL, (double)(mR - mL)), he, coef);
+    }
+
+    // The layers of the next sublayer's top surface are requested as the step
+    // that places its bottom surface begins, where a side has entered a new one.
+    bool newL = false, newR = false;
+    __device__ __forceinline__ void begin() {
+        if (newL) layers((unsigned)(kl - 1) * ncol + colL, qL);
+        if (newR) layers((unsigned)(kr - 1) * ncol + colR, qR);
+    }
+    __device__ __forceinline__ void surface(int ks, unsigned so, double pol, double por, int kol, int kor,
+                                            typename P::He he) {
+        using At = RingAt<NR>;
+        const unsigned tL = threadIdx.x * (unsigned)sizeof(double2), tR = tL + At::kSide;
+        const double2 l0 = sw_ts(r, At::at(tL, kol - 1)), l1 = sw_ts(r, At::at(tL, kol));
+        const double2 r0 = sw_ts(r, At::at(tR, kor - 1)), r1 = sw_ts(r, At::at(tR, kor));
+        const double2 bl = make_double2(interp(pol, l0.x, l1.x), interp(pol, l0.y, l1.y));
+        const double2 br = make_double2(interp(por, r0.x, r1.x), interp(por, r0.y, r1.y));
+        if (ks > 1 && on) {
+            Flux fT = Flux(0), fS = Flux(0);
+            if (he != typename P::He(0)) {
+                // a side's layer moves down by 0 or 1 from one surface to the next
+                typename Ops::Mean mL[2], mR[2];
+                Ops::mean2(pl, kol == kl ? pol : pol + 1.0, qL, mL);
+                Ops::mean2(pr, kor == kr ? por : por + 1.0, qR, mR);
+                fT = flux(tl.x, tr.x, bl.x, br.x, mL[0], mR[0], he);
+                fS = flux(tl.y, tr.y, bl.y, br.y, mL[1], mR[1], he);
+            }
+            FT[so - fstride] = fT;
+            FS[so - fstride] = fS;
+        }
+        newL = kol != kl;
+        newR = kor != kr;
+        tl = bl;
+        tr = br;
+        kl = kol;
+        kr = kor;
+        pl = pol;
+        pr = por;
+    }
+};
 
 // ---------------------------------------------------------------------------
 // The face flux with its reconstruction loads staged one sublayer ahead.

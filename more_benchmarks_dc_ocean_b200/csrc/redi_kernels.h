@@ -100,6 +100,7 @@ struct SweepArgsT {
     const IfcState* ifc;
     const double* pint;
     FaceOutT<P> u, v;
+    double sv_t = 0.0, sv_s = 0.0;  // packed column state: its derivatives over -(rho * rho)
 };
 using SweepArgs = SweepArgsT<PlainPrec>;
 
@@ -278,10 +279,28 @@ struct Band {
 };
 
 cudaError_t launch_column_state(const ColumnStateArgs& cs, cudaStream_t st, Band band = Band{});
+// How a whole step treats T and S (a step's tracers 0 and 1): their fluxes in
+// launches of their own, in the sweep, or in the sweep with the column state
+// packed (a linear equation of state).
+enum class StepForm { kSeparate, kFlux, kFluxPacked };
+// The fluxes go into the sweep when the default forms of the sweep and the
+// face flux are in force, Phase B is not the fused fold, and the flux buffer
+// has a slot for each of the two.
+inline StepForm step_form(int ntr, const CellTuning& t, bool fold, int eos_variant) {
+    if (!(ntr >= 2 && t.sweep_form == 4 && t.flux_staged == 0 && !fold && flux_slots(ntr, t) >= 2))
+        return StepForm::kSeparate;
+    return eos_is_linear(eos_variant) ? StepForm::kFluxPacked : StepForm::kFlux;
+}
 // The column state and the reconstruction of rc's tracers 0 and 1 (T and S,
-// or S and T when ts_swap) in one pass over every column.
+// or S and T when ts_swap) in one pass over every column, as `form` reads them.
 template <class P>
-cudaError_t launch_column_recon(const ColumnStateArgs& cs, const ReconArgsT<P>& rc, int ts_swap, cudaStream_t st);
+cudaError_t launch_column_recon(const ColumnStateArgs& cs, const ReconArgsT<P>& rc, int ts_swap, StepForm form,
+                                cudaStream_t st);
+// The sweep of every face with the fluxes of tracers 0 and 1 of ff (T and S, or
+// S and T when ts_swap) into flux slots 0 and 1.
+template <class P>
+cudaError_t launch_sweep_flux(const SweepArgsT<P>& sw, const FaceFluxArgsT<P>& ff, int ts_swap, StepForm form,
+                              cudaStream_t st, Band band = Band{});
 // Density and dSV/dT, dSV/dS at n points (T, S, p device arrays).
 cudaError_t launch_eos_points(const EosParams& e, int n, const double* T, const double* S, const double* p,
                               double* rho, double* dsv_dt, double* dsv_ds, cudaStream_t st);
@@ -289,8 +308,9 @@ template <class P>
 cudaError_t launch_sweep(const SweepArgsT<P>& sw, cudaStream_t st, Band band = Band{});
 template <class P>
 // recon_from: the first tracer of rc to reconstruct (tracers before it were
-// reconstructed already, by launch_column_recon).
+// reconstructed already, by launch_column_recon). flux_from: 2 when the fluxes
+// of tracers 0 and 1 are in flux slots 0 and 1 already (launch_sweep_flux).
 cudaError_t launch_phase_b(const ReconArgsT<P>& rc, const FaceFluxArgsT<P>& ff, const CellGatherArgsT<P>& cg,
-                           cudaStream_t st, Band band = Band{}, int recon_from = 0);
+                           cudaStream_t st, Band band = Band{}, int recon_from = 0, int flux_from = 0);
 
 }  // namespace redi

@@ -57,10 +57,10 @@ __global__ void __launch_bounds__(128) k_column_state(ColumnStateArgs a, int c0,
     if (col < c1) column_state_item<LdNC>(a, col);
 }
 
-template <class P>
+template <class P, bool TI, bool LIN>
 __global__ void __launch_bounds__(128) k_column_recon(ColumnStateArgs a, ReconArgsT<P> rc, int ts_swap, int ncol) {
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col < ncol) column_recon_item<P, LdNC>(a, rc, ts_swap, col);
+    if (col < ncol) column_recon_item<P, LdNC, TI, LIN>(a, rc, ts_swap, col);
 }
 
 template <class P>
@@ -86,6 +86,32 @@ __global__ void __launch_bounds__(kSweepWinThreads) k_neutral_sweep_w(SweepArgsT
     const int n = block_compact<kSweepWinThreads>(wet, t, list, warp_n);
     if ((int)threadIdx.x < n)
         sweep_item_win<P, LdNC, NR, true>(a, d, list[threadIdx.x], *reinterpret_cast<SweepWin<NR>*>(sweep_win));
+}
+
+// The same sweep with the fluxes of T and S evaluated as its surfaces are
+// placed (FluxSink). Bound by the instructions and dependent chains of a step
+// (480 warp instructions, half of its cycles issue one), then by what it reads
+// through L2. 1440x1080x75 FP64: 7.8 ms for the sweep and both fluxes, against
+// 5.3 + 7.2 ms in launches of their own. On the way there: layers requested at
+// the end of the step before 9.7 ms, unconditionally 9.8, not at all 7.0; the
+// unpacked state (40 bytes an interface) 8.4; 3 blocks per SM 8.4, 5 (a few
+// spilled registers) 8.7; one branch for both sides' means 8.2.
+template <class P, int NR, bool LIN>
+__global__ void __launch_bounds__(kSweepWinThreads, 4) k_sweep_flux(SweepArgsT<P> a, FaceFluxArgsT<P> ff, int ts_swap,
+                                                                    FaceRange r) {
+    extern __shared__ __align__(16) unsigned char sweep_win[];
+    __shared__ int list[kSweepWinThreads];
+    __shared__ int warp_n[kSweepWinThreads / 32];
+    const int d = blockIdx.x & 1;
+    const int t = r.lo[d] + (int)(blockIdx.x >> 1) * blockDim.x + threadIdx.x;
+    const bool wet = t < r.hi[d] && sweep_face_dry<P, LdNC>(a, d, t);
+    const int n = block_compact<kSweepWinThreads>(wet, t, list, warp_n);
+    if ((int)threadIdx.x < n) {
+        using Win = SweepWin<NR, LIN>;
+        Win& ring = *reinterpret_cast<Win*>(sweep_win);
+        const int face = list[threadIdx.x];
+        sweep_item_win<P, LdNC, NR, true, LIN>(a, d, face, ring, FluxSink<P, LdNC, NR, LIN>(ff, ring, ts_swap, d, face));
+    }
 }
 
 template <int NT, class P>
@@ -234,16 +260,22 @@ cudaError_t launch_column_state(const ColumnStateArgs& cs, cudaStream_t st, Band
 }
 
 template <class P>
-cudaError_t launch_column_recon(const ColumnStateArgs& cs, const ReconArgsT<P>& rc, int ts_swap, cudaStream_t st) {
+cudaError_t launch_column_recon(const ColumnStateArgs& cs, const ReconArgsT<P>& rc, int ts_swap, StepForm form,
+                                cudaStream_t st) {
     const int ncol = cs.nx * cs.ny;
+    const unsigned nb = (unsigned)((ncol + 127) / 128);
     launch_begin(K_COLUMN_RECON, st);
-    plain::k_column_recon<P><<<(ncol + 127) / 128, 128, 0, st>>>(cs, rc, ts_swap, ncol);
+    switch (form) {
+        case StepForm::kSeparate: plain::k_column_recon<P, true, false><<<nb, 128, 0, st>>>(cs, rc, ts_swap, ncol); break;
+        case StepForm::kFlux: plain::k_column_recon<P, false, false><<<nb, 128, 0, st>>>(cs, rc, ts_swap, ncol); break;
+        case StepForm::kFluxPacked: plain::k_column_recon<P, false, true><<<nb, 128, 0, st>>>(cs, rc, ts_swap, ncol); break;
+    }
     launch_end(K_COLUMN_RECON, st);
     return cudaGetLastError();
 }
-template cudaError_t launch_column_recon<PlainPrec>(const ColumnStateArgs&, const ReconArgsT<PlainPrec>&, int,
+template cudaError_t launch_column_recon<PlainPrec>(const ColumnStateArgs&, const ReconArgsT<PlainPrec>&, int, StepForm,
                                                     cudaStream_t);
-template cudaError_t launch_column_recon<MixedPrec>(const ColumnStateArgs&, const ReconArgsT<MixedPrec>&, int,
+template cudaError_t launch_column_recon<MixedPrec>(const ColumnStateArgs&, const ReconArgsT<MixedPrec>&, int, StepForm,
                                                     cudaStream_t);
 
 cudaError_t launch_eos_points(const EosParams& e, int n, const double* T, const double* S, const double* p,
@@ -314,6 +346,37 @@ static void launch_gather_rows(const CellGatherArgsT<P>& cg, int tr, int slot, c
            smem, st>>>(cg, tr, slot, c0, c1, ch);
     launch_end(K_CELL_UPDATE, st);
 }
+
+template <class P, bool LIN>
+static cudaError_t launch_sweep_flux_t(const SweepArgsT<P>& sw, const FaceFluxArgsT<P>& ff, int ts_swap,
+                                       const plain::FaceRange& f, unsigned nb, cudaStream_t st) {
+    constexpr int NR = 4;
+    const size_t smem = sizeof(plain::SweepWin<NR, LIN>);  // within the 48 KB that need no opt-in
+    static_assert(sizeof(plain::SweepWin<NR, LIN>) <= 48 * 1024 - 1024, "the ring and the face list");
+    plain::k_sweep_flux<P, NR, LIN><<<2 * nb, plain::kSweepWinThreads, smem, st>>>(sw, ff, ts_swap, f);
+    return cudaSuccess;
+}
+
+template <class P>
+cudaError_t launch_sweep_flux(const SweepArgsT<P>& sw, const FaceFluxArgsT<P>& ff, int ts_swap, StepForm form,
+                              cudaStream_t st, Band band) {
+    const BandRanges r = band_ranges(sw.nx, sw.ny, band);
+    const unsigned nb = face_blocks(r.f);
+    if (nb > 0) {
+        const int kid = P::kMixed ? K_MIXED_SWEEP : K_NEUTRAL_SWEEP;
+        launch_begin(kid, st);
+        const cudaError_t e = form == StepForm::kFluxPacked
+                                  ? launch_sweep_flux_t<P, true>(sw, ff, ts_swap, r.f, nb, st)
+                                  : launch_sweep_flux_t<P, false>(sw, ff, ts_swap, r.f, nb, st);
+        launch_end(kid, st);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaGetLastError();
+}
+template cudaError_t launch_sweep_flux<PlainPrec>(const SweepArgsT<PlainPrec>&, const FaceFluxArgsT<PlainPrec>&, int,
+                                                  StepForm, cudaStream_t, Band);
+template cudaError_t launch_sweep_flux<MixedPrec>(const SweepArgsT<MixedPrec>&, const FaceFluxArgsT<MixedPrec>&, int,
+                                                  StepForm, cudaStream_t, Band);
 
 template <int GNT, class P>
 static void launch_gather(const CellGatherArgsT<P>& cg, int tr, int slot, const BandRanges& r, const CellTuning& tune,
@@ -547,7 +610,7 @@ FoldShape fold_shape(int nz, int ntr) {
 
 template <class P>
 cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& ff, const CellGatherArgsT<P>& cg,
-                           cudaStream_t st, Band band, int recon_from) {
+                           cudaStream_t st, Band band, int recon_from, int flux_from) {
     const BandRanges r = band_ranges(rc_all.nx, rc_all.ny, band);
     // the tracers still to reconstruct: rc_all's from recon_from on
     ReconArgsT<P> rc = rc_all;
@@ -595,9 +658,10 @@ cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& 
     }
     const CellTuning tune = cell_tuning();
     const int group = flux_group(ff.ntr, tune);
+    if (flux_from == 2) launch_gathers<2, P>(cg, 0, r, tune, st);  // T and S: fluxes from the sweep, slots 0 and 1
     if (gather_spans_two(ff.ntr, tune)) {
         // two face-flux launches of 4 tracers (slots 0-3 and 4-7), one gather of 8
-        for (int tr0 = 0; tr0 < ff.ntr; tr0 += 8) {
+        for (int tr0 = flux_from; tr0 < ff.ntr; tr0 += 8) {
             launch_flux<4, P>(ff, tr0, r, tune, st);
             if (tr0 + 4 < ff.ntr) {
                 FaceFluxArgsT<P> f2 = ff;
@@ -608,7 +672,7 @@ cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& 
         }
         return cudaGetLastError();
     }
-    for (int tr0 = 0; tr0 < ff.ntr; tr0 += group) {
+    for (int tr0 = flux_from; tr0 < ff.ntr; tr0 += group) {
         switch (group) {
             case 8: launch_flux<8, P>(ff, tr0, r, tune, st); launch_gathers<8, P>(cg, tr0, r, tune, st); break;
             case 4: launch_flux<4, P>(ff, tr0, r, tune, st); launch_gathers<4, P>(cg, tr0, r, tune, st); break;
@@ -622,10 +686,10 @@ cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& 
 template cudaError_t launch_sweep<PlainPrec>(const SweepArgsT<PlainPrec>&, cudaStream_t, Band);
 template cudaError_t launch_sweep<MixedPrec>(const SweepArgsT<MixedPrec>&, cudaStream_t, Band);
 template cudaError_t launch_phase_b<PlainPrec>(const ReconArgsT<PlainPrec>&, const FaceFluxArgsT<PlainPrec>&,
-                                               const CellGatherArgsT<PlainPrec>&, cudaStream_t, Band, int);
+                                               const CellGatherArgsT<PlainPrec>&, cudaStream_t, Band, int, int);
 template FoldShape fold_shape<PlainPrec>(int, int);
 template FoldShape fold_shape<MixedPrec>(int, int);
 template cudaError_t launch_phase_b<MixedPrec>(const ReconArgsT<MixedPrec>&, const FaceFluxArgsT<MixedPrec>&,
-                                               const CellGatherArgsT<MixedPrec>&, cudaStream_t, Band, int);
+                                               const CellGatherArgsT<MixedPrec>&, cudaStream_t, Band, int, int);
 
 }  // namespace redi

@@ -553,6 +553,41 @@ def test_whole_step_call_matches_two_calls(redi_lib, oracle_lib, case, precision
             _assert_exact(f"{case} whole-step call vs oracle tracer {n}", a, b)
 
 
+@pytest.mark.parametrize("nx,ny,nz,npas,eos,swap,walls,precision",
+                         [(33, 21, 25, 0, 1, False, True, 0), (17, 130, 9, 0, 1, True, False, 0), (40, 12, 1, 1, 1, False, True, 0),
+                          (29, 19, 2, 0, 2, True, True, 0), (45, 27, 30, 3, 2, False, False, 0), (31, 23, 12, 2, 4, False, True, 1),
+                          (33, 21, 26, 1, 1, True, True, 1), (8, 6, 5, 0, 1, False, True, 0)])
+def test_whole_step_coefficients_and_fluxes(redi_lib, nx, ny, nz, npas, eos, swap, walls, precision):
+    """The whole step with the fluxes of T and S inside the sweep, with the packed column state (linear
+    equation of state) and without: tracers and coefficients of the two calls bit for bit."""
+    R = redi_lib
+    p = inputs.make_problem(nx, ny, nz, n_passive=npas, seed=nz)
+    if swap:
+        p.tracers[0], p.tracers[1] = p.tracers[1], p.tracers[0]
+        p.idx_temperature, p.idx_salinity = p.idx_salinity, p.idx_temperature
+    out = []
+    for combined in (False, True):
+        dp = R.to_device(p)
+        dp.eos.variant = eos
+        bc = dp.bc if walls else R.OceanBC(west=0, east=0, south=0, north=0)
+        redi = R.make_redi(dp, R.MIXED if precision else R.FP64)
+        for _ in range(2):
+            if combined:
+                assert R.redi_step(dp.grid, dp.metrics, dp.eos, redi, dp.ms, dp.dt, dp.khtr_u_ext, dp.khtr_v_ext, bc) == R.OK
+            else:
+                assert R.redi_calc_coeffs(dp.grid, dp.metrics, dp.eos, redi, dp.ms) == R.OK
+                assert R.redi_apply_flux(dp.grid, dp.metrics, redi, dp.ms, dp.dt, dp.khtr_u_ext, dp.khtr_v_ext, bc) == R.OK
+        torch.cuda.synchronize()
+        assert redi.error_count() == 0
+        got = {f"tracer {n}": t.cpu().numpy() for n, t in enumerate(dp.ms.tracers)}
+        if not precision:
+            got.update({k: v.cpu().numpy() for k, v in redi.coeffs().items()})
+        out.append(got)
+        redi.destroy()
+    for k, v in out[0].items():
+        _assert_exact(k, out[1][k], v)
+
+
 def test_whole_step_call_gates(redi_lib):
     """redi_b200_step keeps each phase's gates: a disabled handle is SKIPPED."""
     R = redi_lib
