@@ -365,7 +365,7 @@ REDI_B200_API int redi_b200_halo_copy(double* const* fields, int nfields, int nx
                                       double* buf, int to_buf, void* stream);
 
 /* ---------------------------------------------------------------------------
- * Many independent regional domains stepped by one persistent kernel (no
+ * Many independent regional domains stepped together (no
  * counterpart in the reference, whose driver steps one domain per call). The
  * step of every domain (redi_calc_coeffs then redi_apply_flux for all of its
  * tracers) is cut into tiles of columns, faces and cells; one grid of resident
@@ -422,6 +422,16 @@ REDI_B200_API int redi_b200_batch_status(const redi_b200_batch* b, int* status, 
 REDI_B200_API int redi_b200_batch_set_tuning(redi_b200_batch* b, int tile_bx, int tile_by, int chunk, int occupancy);
 REDI_B200_API int redi_b200_batch_get_tuning(const redi_b200_batch* b, int* tile_bx, int* tile_by, int* chunk,
                                              int* occupancy, int* grid);
+
+/* Form of the step: one persistent kernel over the whole work queue, or the
+ * handle API's launches for every domain on a few streams (the default); both
+ * are captured in the graph. Results do not depend on it. The accounting below
+ * is the persistent kernel's: a step with it on takes that form, and the launch
+ * shape above is that kernel's. get returns the form in force. */
+#define REDI_B200_BATCH_PERSISTENT 1
+#define REDI_B200_BATCH_LAUNCHES 2
+REDI_B200_API int redi_b200_batch_set_form(redi_b200_batch* b, int form);
+REDI_B200_API int redi_b200_batch_get_form(const redi_b200_batch* b);
 
 /* Per-stage accounting of the last step (off by default): with on != 0 the
  * kernel sums, per stage kind (0 column state, 1 neutral sweep, 2 tracer

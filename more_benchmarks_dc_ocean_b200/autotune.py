@@ -288,11 +288,12 @@ K_DOMAIN_PERSISTENT = 8
 
 def tune_batch(batch, candidates: Optional[Iterable[Tuple[int, int, int]]] = None, reps: int = 2,
                stream=None) -> dict:
-    """Time whole batch steps for every (bx, by, chunk, occupancy) candidate and keep the fastest.
+    """Time whole batch steps for every (bx, by, chunk, occupancy) candidate of the persistent kernel and
+    for the launches per domain (which have no shape to choose); keep the fastest.
 
     The persistent kernel runs every stage of every domain, so the candidate is
     compared on the full step (its tracers are advanced in place). Returns
-    {"best": (bx, by, chunk, occupancy), "ms": {candidate: ms per step}}.
+    {"best": (bx, by, chunk, occupancy), "form": the form kept, "ms": {candidate: ms per step}}.
     """
     import torch
 
@@ -301,9 +302,8 @@ def tune_batch(batch, candidates: Optional[Iterable[Tuple[int, int, int]]] = Non
     L = _bind(R.lib())
     cands = list(candidates) if candidates is not None else [(bx, by, c, o) for (bx, by) in BATCH_TILES
                                                              for c in CHUNKS for o in BATCH_OCCUPANCY]
-    times = {}
-    for cand in cands:
-        batch.set_tuning(cand[:2], cand[2], cand[3] if len(cand) > 3 else 0)
+
+    def timed():
         batch.step(1, stream)  # graph capture + warm-up
         torch.cuda.synchronize()
         L.redi_b200_profile_begin()
@@ -311,8 +311,20 @@ def tune_batch(batch, candidates: Optional[Iterable[Tuple[int, int, int]]] = Non
         kt = (C.c_double * R.lib().redi_b200_kernel_count())()
         kc = (C.c_ulonglong * R.lib().redi_b200_kernel_count())()
         R._check(L.redi_b200_profile_end(kt, kc, len(kt)))
-        times[cand] = kt[K_DOMAIN_PERSISTENT] / max(1, kc[K_DOMAIN_PERSISTENT])
+        return kt[K_DOMAIN_PERSISTENT] / max(1, kc[K_DOMAIN_PERSISTENT])
+
+    times = {}
+    batch.set_form(R.BATCH_PERSISTENT)
+    for cand in cands:
+        batch.set_tuning(cand[:2], cand[2], cand[3] if len(cand) > 3 else 0)
+        times[cand] = timed()
     best = min(times, key=times.get)
     batch.set_tuning(best[:2], best[2], best[3] if len(best) > 3 else 0)
-    return {"best": best, "ms": {"x".join(map(str, k[:2])) + f"/ch{k[2]}" + (f"/occ{k[3]}" if len(k) > 3 else ""):
-                                 round(v, 4) for k, v in times.items()}}
+    ms = {"x".join(map(str, k[:2])) + f"/ch{k[2]}" + (f"/occ{k[3]}" if len(k) > 3 else ""): round(v, 4)
+          for k, v in times.items()}
+    batch.set_form(R.BATCH_LAUNCHES)
+    t = timed()
+    ms["launches"] = round(t, 4)
+    if t > times[best]:
+        batch.set_form(R.BATCH_PERSISTENT)
+    return {"best": best, "form": batch.get_form(), "ms": ms}

@@ -77,6 +77,8 @@ struct FaceInT {
 using FaceOut = FaceOutT<PlainPrec>;
 using FaceIn = FaceInT<PlainPrec>;
 
+// `stop` in the arguments of a launch (may be null): a device word that makes
+// the launch do nothing once it is not zero (a batch whose step was given up).
 struct ColumnStateArgs {
     int nx, ny, nz;
     EosParams eos;
@@ -89,6 +91,7 @@ struct ColumnStateArgs {
     // is wet is never read by the sweep, and is not computed
     const double* wet_u = nullptr;
     const double* wet_v = nullptr;
+    const int* stop = nullptr;  // a launch does nothing once *stop != 0
 };
 
 template <class P>
@@ -101,6 +104,7 @@ struct SweepArgsT {
     const double* pint;
     FaceOutT<P> u, v;
     double sv_t = 0.0, sv_s = 0.0;  // packed column state: its derivatives over -(rho * rho)
+    const int* stop = nullptr;
 };
 using SweepArgs = SweepArgsT<PlainPrec>;
 
@@ -115,6 +119,7 @@ struct ReconArgsT {
     // are dry is never read by the face flux, and is not reconstructed
     const uint8_t* dry_u = nullptr;
     const uint8_t* dry_v = nullptr;
+    const int* stop = nullptr;
 };
 using ReconArgs = ReconArgsT<PlainPrec>;
 
@@ -137,6 +142,7 @@ struct FaceFluxArgsT {
     typename P::Flux* Fu;             // [slot][ns-1][(nx+1)*ny]
     typename P::Flux* Fv;             // [slot][ns-1][nx*(ny+1)]
     int fslot0 = 0;                   // slot of the launch's first tracer
+    const int* stop = nullptr;
 };
 using FaceFluxArgs = FaceFluxArgsT<PlainPrec>;
 
@@ -152,6 +158,7 @@ struct CellGatherArgsT {
     double* htr[kMaxTracers];         // updated tracers
     const double* htr_in[kMaxTracers];  // pre-step tracers (the same arrays for an in-place update)
     int* err;                         // device error word (fluxes out of order), may be null
+    const int* stop = nullptr;
 };
 using CellGatherArgs = CellGatherArgsT<PlainPrec>;
 
@@ -216,6 +223,15 @@ void launch_end(int kid, cudaStream_t st);
 // Adds n launches of kernel kid to the counter without timing them (CUDA graph
 // replays, whose launches happen inside the graph).
 void count_launches(int kid, unsigned long long n);
+// While one lives, the calling thread's launches are neither counted nor timed
+// but tallied here (a step captured into a graph, or timed as a whole).
+struct LaunchTally {
+    unsigned long long n[K_NUM] = {};
+    LaunchTally();
+    ~LaunchTally();
+    LaunchTally(const LaunchTally&) = delete;
+    LaunchTally& operator=(const LaunchTally&) = delete;
+};
 
 // Launch shape of Phase B: the cell gather's bx x by tile of columns per
 // block (bx * by <= 128) and vertical chunk (layers per pass, 4, 8 or 16),
@@ -310,7 +326,9 @@ template <class P>
 // recon_from: the first tracer of rc to reconstruct (tracers before it were
 // reconstructed already, by launch_column_recon). flux_from: 2 when the fluxes
 // of tracers 0 and 1 are in flux slots 0 and 1 already (launch_sweep_flux).
+// pairs_only: the flux buffer has two slots, and the fused fold is left out.
 cudaError_t launch_phase_b(const ReconArgsT<P>& rc, const FaceFluxArgsT<P>& ff, const CellGatherArgsT<P>& cg,
-                           cudaStream_t st, Band band = Band{}, int recon_from = 0, int flux_from = 0);
+                           cudaStream_t st, Band band = Band{}, int recon_from = 0, int flux_from = 0,
+                           bool pairs_only = false);
 
 }  // namespace redi

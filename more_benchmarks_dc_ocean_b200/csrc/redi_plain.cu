@@ -53,18 +53,21 @@ struct FaceRange {
 };
 
 __global__ void __launch_bounds__(128) k_column_state(ColumnStateArgs a, int c0, int c1) {
+    if (a.stop && *a.stop) return;
     const int col = c0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (col < c1) column_state_item<LdNC>(a, col);
 }
 
 template <class P, bool TI, bool LIN>
 __global__ void __launch_bounds__(128) k_column_recon(ColumnStateArgs a, ReconArgsT<P> rc, int ts_swap, int ncol) {
+    if (a.stop && *a.stop) return;
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col < ncol) column_recon_item<P, LdNC, TI, LIN>(a, rc, ts_swap, col);
 }
 
 template <class P>
 __global__ void __launch_bounds__(128) k_neutral_sweep(SweepArgsT<P> a, FaceRange r) {
+    if (a.stop && *a.stop) return;
     const int d = blockIdx.x & 1;  // blocks alternate between u and v faces, as in k_face_flux
     const int t = r.lo[d] + (int)(blockIdx.x >> 1) * blockDim.x + threadIdx.x;
     if (t < r.hi[d]) sweep_item<P, LdNC, true>(a, d, t);
@@ -77,6 +80,7 @@ __global__ void __launch_bounds__(128) k_neutral_sweep(SweepArgsT<P> a, FaceRang
 // the sweeps of a block with land run in as few warps as its wet faces fill.
 template <class P, int NR>
 __global__ void __launch_bounds__(kSweepWinThreads) k_neutral_sweep_w(SweepArgsT<P> a, FaceRange r) {
+    if (a.stop && *a.stop) return;
     extern __shared__ __align__(16) unsigned char sweep_win[];
     __shared__ int list[kSweepWinThreads];
     __shared__ int warp_n[kSweepWinThreads / 32];
@@ -99,6 +103,7 @@ __global__ void __launch_bounds__(kSweepWinThreads) k_neutral_sweep_w(SweepArgsT
 template <class P, int NR, bool LIN>
 __global__ void __launch_bounds__(kSweepWinThreads, 4) k_sweep_flux(SweepArgsT<P> a, FaceFluxArgsT<P> ff, int ts_swap,
                                                                     FaceRange r) {
+    if (a.stop && *a.stop) return;
     extern __shared__ __align__(16) unsigned char sweep_win[];
     __shared__ int list[kSweepWinThreads];
     __shared__ int warp_n[kSweepWinThreads / 32];
@@ -116,6 +121,7 @@ __global__ void __launch_bounds__(kSweepWinThreads, 4) k_sweep_flux(SweepArgsT<P
 
 template <int NT, class P>
 __global__ void __launch_bounds__(128) k_tracer_recon(ReconArgsT<P> a, int c0, int nb) {
+    if (a.stop && *a.stop) return;
     recon_item<NT, P, LdNC>(a, blockIdx.x * blockDim.x + threadIdx.x, c0, nb);
 }
 
@@ -128,6 +134,7 @@ __global__ void __launch_bounds__(128) k_tracer_recon(ReconArgsT<P> a, int c0, i
 // with no face left, return at once.
 template <int NT, class P>
 __global__ void __launch_bounds__(128) k_face_flux(FaceFluxArgsT<P> a, int tr0, FaceRange r) {
+    if (a.stop && *a.stop) return;
     __shared__ int list[128];
     __shared__ int warp_n[4];
     const int d = blockIdx.x & 1;
@@ -142,6 +149,7 @@ __global__ void __launch_bounds__(128) k_face_flux(FaceFluxArgsT<P> a, int tr0, 
 // in shared memory (flux_item_ring); the same block order.
 template <int NT, class P>
 __global__ void __launch_bounds__(kFluxThreads) k_face_flux_r(FaceFluxArgsT<P> a, int tr0, FaceRange r) {
+    if (a.stop && *a.stop) return;
     extern __shared__ __align__(16) unsigned char ring[];
     __shared__ int list[kFluxThreads];
     __shared__ int warp_n[kFluxThreads / 32];
@@ -155,6 +163,7 @@ __global__ void __launch_bounds__(kFluxThreads) k_face_flux_r(FaceFluxArgsT<P> a
 
 template <int NT, class P>
 __global__ void __launch_bounds__(kFluxThreads) k_face_flux_s(FaceFluxArgsT<P> a, int tr0, FaceRange r) {
+    if (a.stop && *a.stop) return;
     extern __shared__ __align__(16) unsigned char stage[];
     double* sti = reinterpret_cast<double*>(stage);
     double2* spp = reinterpret_cast<double2*>(stage + FluxStage<NT, P>::ti_doubles * sizeof(double));
@@ -165,6 +174,7 @@ __global__ void __launch_bounds__(kFluxThreads) k_face_flux_s(FaceFluxArgsT<P> a
 
 template <int NT, int CH, class P>
 __global__ void __launch_bounds__(128) k_cell_gather(CellGatherArgsT<P> a, int tr0, int fslot, int j0, int j1) {
+    if (a.stop && *a.stop) return;
     const int j = j0 + blockIdx.y * blockDim.y + threadIdx.y;
     // sublayers fetched per round trip: 3 with 4-layer chunks, 4 with deeper chunks (measured)
     if (j < j1) gather_item<NT, CH, P, LdNC, (CH <= 4 ? 3 : 4)>(a, blockIdx.x * blockDim.x + threadIdx.x, j, tr0, fslot);
@@ -176,6 +186,7 @@ __global__ void __launch_bounds__(128) k_cell_gather(CellGatherArgsT<P> a, int t
 template <int NT, int CH, class P, int U = 0, bool PIPE = false>
 __global__ void __launch_bounds__(kGatherThreads) k_cell_gather_s(CellGatherArgsT<P> a, int tr0, int fslot, int j0,
                                                                   int j1) {
+    if (a.stop && *a.stop) return;
     __shared__ double acc[CH * NT * kGatherThreads];
     const int tid = threadIdx.x + blockDim.x * threadIdx.y;
     const int j = j0 + blockIdx.y * blockDim.y + threadIdx.y;
@@ -189,6 +200,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_cell_gather_s(CellGatherArgs
 template <int NT, class P, int U>
 __global__ void __launch_bounds__(kGatherRowThreads) k_cell_gather_rows(CellGatherArgsT<P> a, int tr0, int fslot, int c0,
                                                                         int c1, int ch) {
+    if (a.stop && *a.stop) return;
     extern __shared__ __align__(16) char rowsum[];
     __shared__ int2 walk[4 * kGatherRowThreads];  // per face: the warp's and the lane's next sublayer
     gather_item_rows<NT, P, LdNC, U>(a, c0 + blockIdx.x * kGatherRowThreads + threadIdx.x, c1, tr0, fslot, ch,
@@ -610,7 +622,7 @@ FoldShape fold_shape(int nz, int ntr) {
 
 template <class P>
 cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& ff, const CellGatherArgsT<P>& cg,
-                           cudaStream_t st, Band band, int recon_from, int flux_from) {
+                           cudaStream_t st, Band band, int recon_from, int flux_from, bool pairs_only) {
     const BandRanges r = band_ranges(rc_all.nx, rc_all.ny, band);
     // the tracers still to reconstruct: rc_all's from recon_from on
     ReconArgsT<P> rc = rc_all;
@@ -621,7 +633,7 @@ cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& 
         rc.ti = rc_all.ti + (size_t)recon_from * ncol * (rc_all.nz + 1);
         rc.ppm = rc_all.ppm + (size_t)recon_from * ncol * rc_all.nz;
     }
-    const FoldShape fs = fold_shape<P>(rc.nz, ff.ntr);
+    const FoldShape fs = pairs_only ? FoldShape{0, 0} : fold_shape<P>(rc.nz, ff.ntr);
     if (fs.nt > 0) {
         if (r.c1 > r.c0 && rc.ntr > 0) {
             launch_recon<P>(rc, r, st);
@@ -656,7 +668,11 @@ cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& 
     if (r.c1 > r.c0 && rc.ntr > 0) {
         launch_recon<P>(rc, r, st);
     }
-    const CellTuning tune = cell_tuning();
+    CellTuning tune = cell_tuning();
+    if (pairs_only) {
+        tune.group = min(tune.group, 2);
+        tune.gather_tracers = 2;
+    }
     const int group = flux_group(ff.ntr, tune);
     if (flux_from == 2) launch_gathers<2, P>(cg, 0, r, tune, st);  // T and S: fluxes from the sweep, slots 0 and 1
     if (gather_spans_two(ff.ntr, tune)) {
@@ -686,10 +702,10 @@ cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& 
 template cudaError_t launch_sweep<PlainPrec>(const SweepArgsT<PlainPrec>&, cudaStream_t, Band);
 template cudaError_t launch_sweep<MixedPrec>(const SweepArgsT<MixedPrec>&, cudaStream_t, Band);
 template cudaError_t launch_phase_b<PlainPrec>(const ReconArgsT<PlainPrec>&, const FaceFluxArgsT<PlainPrec>&,
-                                               const CellGatherArgsT<PlainPrec>&, cudaStream_t, Band, int, int);
+                                               const CellGatherArgsT<PlainPrec>&, cudaStream_t, Band, int, int, bool);
 template FoldShape fold_shape<PlainPrec>(int, int);
 template FoldShape fold_shape<MixedPrec>(int, int);
 template cudaError_t launch_phase_b<MixedPrec>(const ReconArgsT<MixedPrec>&, const FaceFluxArgsT<MixedPrec>&,
-                                               const CellGatherArgsT<MixedPrec>&, cudaStream_t, Band, int, int);
+                                               const CellGatherArgsT<MixedPrec>&, cudaStream_t, Band, int, int, bool);
 
 }  // namespace redi

@@ -486,6 +486,7 @@ def step(dp: DeviceProblem, redi: OceanRedi, nsteps: int = 1, stream=None) -> No
 # Many domains in one persistent launch (no counterpart in the reference)
 # ---------------------------------------------------------------------------
 STATUS_TIMEOUT = 1
+BATCH_PERSISTENT, BATCH_LAUNCHES = 1, 2
 STAGE_NAMES = ("column_state", "neutral_sweep", "tracer_recon")
 
 
@@ -507,6 +508,8 @@ def _batch_lib() -> C.CDLL:
         L.redi_b200_batch_set_tuning.argtypes = [vp, C.c_int, C.c_int, C.c_int, C.c_int]
         L.redi_b200_batch_get_tuning.argtypes = [vp, _ip, _ip, _ip, _ip, _ip]
         L.redi_b200_batch_set_accounting.argtypes = [vp, C.c_int]
+        L.redi_b200_batch_set_form.argtypes = [vp, C.c_int]
+        L.redi_b200_batch_get_form.argtypes = [vp]
         L.redi_b200_batch_stage_times.argtypes = [vp, _dp, _dp, C.POINTER(C.c_longlong)]
         L.redi_b200_batch_updates.argtypes = [vp]
         L.redi_b200_batch_updates.restype = C.c_longlong
@@ -526,7 +529,8 @@ def stage_name(stage: int) -> str:
 
 
 class RediBatch:
-    """Independent regional domains stepped together by one persistent kernel.
+    """Independent regional domains stepped together: one persistent kernel, or one graph of every
+    domain's launches (set_form).
 
     ``domains`` are ``DeviceProblem``s (per-face diffusivities required); their
     tensors must stay alive while the batch exists, their device addresses are
@@ -584,6 +588,15 @@ class RediBatch:
         _check(_batch_lib().redi_b200_batch_get_tuning(self._h, C.byref(bx), C.byref(by), C.byref(ch), C.byref(occ),
                                                        C.byref(grid)))
         return {"tile": (bx.value, by.value), "chunk": ch.value, "occupancy": occ.value, "grid": grid.value}
+
+    def set_form(self, form: int) -> None:
+        """BATCH_PERSISTENT (one kernel over the work queue) or BATCH_LAUNCHES (every domain's launches
+        on a few streams, the default); results do not depend on it."""
+        _check(_batch_lib().redi_b200_batch_set_form(self._h, int(form)))
+
+    def get_form(self) -> int:
+        """The form a step takes now: BATCH_PERSISTENT or BATCH_LAUNCHES."""
+        return _check(_batch_lib().redi_b200_batch_get_form(self._h))
 
     def set_accounting(self, on: bool = True) -> None:
         _check(_batch_lib().redi_b200_batch_set_accounting(self._h, int(bool(on))))

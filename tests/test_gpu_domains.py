@@ -146,3 +146,60 @@ def test_batch_rejects_bad_arguments(redi_lib):
     dp.khtr_u_ext = None
     with pytest.raises(R.RediError, match="NULL"):
         R.RediBatch([dp])
+
+
+@pytest.mark.parametrize("precision,graph,swap", [(0, True, False), (0, False, True), (1, True, False)])
+def test_batch_forms_identical(redi_lib, precision, graph, swap):
+    """The persistent kernel and the launches per domain give the same bits over three steps, with T and S
+    in either order, and a step may change form."""
+    R = redi_lib
+    ps = _domains()
+    if swap:
+        for p in ps[:2]:
+            p.tracers[0], p.tracers[1] = p.tracers[1], p.tracers[0]
+            p.idx_temperature, p.idx_salinity = p.idx_salinity, p.idx_temperature
+        ps[2].tracers[1], ps[2].tracers[4] = ps[2].tracers[4], ps[2].tracers[1]
+        ps[2].idx_salinity = 5
+    out = []
+    for forms in ((R.BATCH_PERSISTENT,) * 3, (R.BATCH_LAUNCHES, R.BATCH_PERSISTENT, R.BATCH_LAUNCHES)):
+        dps = [R.to_device(p) for p in ps]
+        b = R.RediBatch(dps, precision=precision, use_graph=graph)
+        for f in forms:
+            b.set_form(f)
+            assert b.get_form() == f
+            b.step()
+            st = b.status()
+            assert st["status"] == 0 and st["bad"] == 0, st
+        torch.cuda.synchronize()
+        b.destroy()
+        out.append([[t.cpu().numpy() for t in dp.ms.tracers] for dp in dps])
+    for p, x, y in zip(ps, out[1], out[0]):
+        for n in range(len(x)):
+            _assert_exact(f"{p.name} tracer {n}", x[n], y[n])
+
+
+def test_batch_launches_time_out_on_a_held_domain(redi_lib):
+    """The launches per domain: a held domain ends the step with the status, no tracer is touched, and the
+    next step runs."""
+    R = redi_lib
+    ps = _domains()[:3]
+    dps = [R.to_device(p) for p in ps]
+    b = R.RediBatch(dps)
+    b.set_form(R.BATCH_LAUNCHES)
+    b.set_wait_limit(20_000_000)  # 20 ms
+    b.hold(1)
+    b.step()
+    st = b.status()
+    assert st["status"] == R.STATUS_TIMEOUT and st["domain"] == 1 and st["stage"] == 0, st
+    for p, dp in zip(ps, dps):
+        for a, t in zip(p.tracers, dp.ms.tracers):
+            _assert_exact(f"{p.name} untouched", t.cpu().numpy(), a)
+    b.hold(1, False)
+    b.step()
+    assert b.status()["status"] == 0
+    got = [[t.cpu().numpy() for t in dp.ms.tracers] for dp in dps]
+    b.destroy()
+    for p, g in zip(ps, got):
+        ref = _handle_run(R, p, 1)
+        for n, (a, c) in enumerate(zip(g, ref)):
+            _assert_exact(f"{p.name} tracer {n}", a, c)
