@@ -170,6 +170,7 @@ redi::FaceFluxArgsT<P> flux_args(const PhaseBInputs<P>& in, const PhaseBBuffers<
     ff.ti = reinterpret_cast<double*>(base);
     ff.ppm = reinterpret_cast<typename P::Ppm*>(base + redi::recon_ppm_offset(in.nx, in.ny, in.nz, nt));
     ff.Fu = reinterpret_cast<Flux*>(base + buf.recon);
+    ff.slots = buf.group;
     ff.Fv = ff.Fu + (size_t)buf.group * (size_t)(2 * in.nz + 1) * (size_t)(in.nx + 1) * in.ny;
     return ff;
 }

@@ -421,7 +421,8 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
                               up256(nv * ns * sizeof(Ko)) * 2 + up256(nu * (ns - 1) * sizeof(He)) +
                               up256(nv * (ns - 1) * sizeof(He)) + up256(nu) + up256(nv);
         const size_t a_b = redi::phase_a_scratch(nx, ny, nz);
-        const size_t rb = redi::recon_bytes<P>(nx, ny, nz, ntr), fb = redi::flux_bytes<P>(nx, ny, nz, 2);
+        const int slots = 2 * std::min(redi::kPairsPerLaunch, (ntr + 1) / 2);
+        const size_t rb = redi::recon_bytes<P>(nx, ny, nz, ntr), fb = redi::flux_bytes<P>(nx, ny, nz, slots);
         // Phase A's state beside Phase B's buffers: the sweep that evaluates the fluxes needs both
         const size_t scratch = up256(rb) + up256(fb) + a_b;
         char* base = nullptr;
@@ -474,7 +475,8 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
         ff.v = redi::FaceInT<P>{v.PoL, v.PoR, v.KoL, v.KoR, v.hEff, v.dry};
         ff.ti = d.rc.ti; ff.ppm = d.rc.ppm;
         ff.Fu = (typename P::Flux*)(sc + up256(rb));
-        ff.Fv = ff.Fu + (size_t)2 * (2 * nz + 1) * nu;
+        ff.slots = slots;
+        ff.Fv = ff.Fu + (size_t)slots * (2 * nz + 1) * nu;
         auto& cg = d.cg;
         cg.nx = nx; cg.ny = ny; cg.nz = nz; cg.ntr = ntr; cg.nghost = ff.nghost; cg.nxp = ff.nxp; cg.nyp = ff.nyp;
         cg.wall_w = walls[0]; cg.wall_e = walls[1]; cg.wall_s = walls[2]; cg.wall_n = walls[3];

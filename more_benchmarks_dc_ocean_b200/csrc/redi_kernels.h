@@ -142,6 +142,7 @@ struct FaceFluxArgsT {
     typename P::Flux* Fu;             // [slot][ns-1][(nx+1)*ny]
     typename P::Flux* Fv;             // [slot][ns-1][nx*(ny+1)]
     int fslot0 = 0;                   // slot of the launch's first tracer
+    int slots = 0;                    // slots of the flux buffer
     const int* stop = nullptr;
 };
 using FaceFluxArgs = FaceFluxArgsT<PlainPrec>;
@@ -262,8 +263,18 @@ inline bool gather_spans_two(int ntr, const CellTuning& t) {
     return !t.gather_rows && t.gather_tracers >= 8 && flux_group(ntr, t) == 4 && ntr > 4 && t.gather_smem && t.chunk == 4 &&
            t.bx * t.by == 128;
 }
+// Tracer pairs whose face fluxes, and then gathers, share a launch: the default
+// forms (groups of two, the row gather) read the coefficients they share from
+// L2 when the pairs of a tile run side by side.
+constexpr int kPairsPerLaunch = 4;
+inline bool pairs_share_launches(int ntr, const CellTuning& t) {
+    return t.flux_staged == 0 && t.gather_rows && flux_group(ntr, t) == 2;
+}
 // Slots of the flux buffer Phase B needs for ntr tracers.
-inline int flux_slots(int ntr, const CellTuning& t) { return gather_spans_two(ntr, t) ? 8 : flux_group(ntr, t); }
+inline int flux_slots(int ntr, const CellTuning& t) {
+    if (pairs_share_launches(ntr, t)) return 2 * ((ntr + 1) / 2 < kPairsPerLaunch ? (ntr + 1) / 2 : kPairsPerLaunch);
+    return gather_spans_two(ntr, t) ? 8 : flux_group(ntr, t);
+}
 
 // Phase B as one fused face-flux + fold pass (redi_fold.cuh) instead of the
 // face-flux / cell-gather pair: enable, tile rows (1 or 2) and tracers per
@@ -326,9 +337,9 @@ template <class P>
 // recon_from: the first tracer of rc to reconstruct (tracers before it were
 // reconstructed already, by launch_column_recon). flux_from: 2 when the fluxes
 // of tracers 0 and 1 are in flux slots 0 and 1 already (launch_sweep_flux).
-// pairs_only: the flux buffer has two slots, and the fused fold is left out.
+// no_fold: the fused fold is left out. ff.slots bounds the tracers per launch.
 cudaError_t launch_phase_b(const ReconArgsT<P>& rc, const FaceFluxArgsT<P>& ff, const CellGatherArgsT<P>& cg,
                            cudaStream_t st, Band band = Band{}, int recon_from = 0, int flux_from = 0,
-                           bool pairs_only = false);
+                           bool no_fold = false);
 
 }  // namespace redi

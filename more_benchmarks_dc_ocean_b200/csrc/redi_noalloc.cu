@@ -174,7 +174,7 @@ int redi_b200_opt_launch_noalloc(const int* nx_, const int* ny_, const int* nz_,
     ff.dy_cu = dy_cu; ff.dx_cv = dx_cv; ff.idxCu = idxCu; ff.idyCv = idyCv;
     ff.u = redi::FaceIn{uPoL, uPoR, uKoL, uKoR, uhEff, udry};
     ff.v = redi::FaceIn{vPoL, vPoR, vKoL, vKoR, vhEff, vdry};
-    ff.ti = r.ti; ff.ppm = r.ppm;
+    ff.ti = r.ti; ff.ppm = r.ppm; ff.slots = 2;
     ff.Fu = reinterpret_cast<double*>(data + ti_b + ppm_b);
     ff.Fv = reinterpret_cast<double*>(data + ti_b + ppm_b + fu_b);
     redi::CellGatherArgs cg{};

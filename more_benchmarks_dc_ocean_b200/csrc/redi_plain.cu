@@ -132,13 +132,22 @@ __global__ void __launch_bounds__(128) k_tracer_recon(ReconArgsT<P> a, int c0, i
 // The block's faces that need a flux (not walls, not dry) are compacted onto
 // its leading threads in face order; the others walk as stand-ins or, in warps
 // with no face left, return at once.
-template <int NT, class P>
-__global__ void __launch_bounds__(128) k_face_flux(FaceFluxArgsT<P> a, int tr0, FaceRange r) {
+// PAIRS: `pairs` groups of NT tracers in one launch, the blocks of one tile of
+// faces side by side.
+template <int NT, class P, bool PAIRS>
+__global__ void __launch_bounds__(128) k_face_flux(FaceFluxArgsT<P> a, int tr0, int pairs, FaceRange r) {
     if (a.stop && *a.stop) return;
     __shared__ int list[128];
     __shared__ int warp_n[4];
-    const int d = blockIdx.x & 1;
-    const int t = r.lo[d] + (int)(blockIdx.x >> 1) * blockDim.x + threadIdx.x;
+    unsigned b = blockIdx.x;
+    if constexpr (PAIRS) {
+        b = blockIdx.x / pairs;
+        const int g = NT * (int)(blockIdx.x - b * pairs);
+        tr0 += g;
+        a.fslot0 += g;
+    }
+    const int d = b & 1;
+    const int t = r.lo[d] + (int)(b >> 1) * blockDim.x + threadIdx.x;
     const int n = block_compact<128>(flux_face_valid(a, d, t, r.hi[d]), t, list, warp_n);
     flux_item<NT, P, LdNC>(a, d, (int)threadIdx.x < n ? list[threadIdx.x] : r.hi[d], tr0, r.hi[d]);
 }
@@ -197,13 +206,21 @@ __global__ void __launch_bounds__(kGatherThreads) k_cell_gather_s(CellGatherArgs
 
 // The gather with a warp on whole rows of sublayers (gather_item_rows): one
 // warp per block, cells [c0, c1) in column order, so a ragged nx wastes no lane.
-template <int NT, class P, int U>
+// PAIRS: `pairs` groups of NT tracers, the blocks of one warp of cells side by side.
+template <int NT, class P, int U, bool PAIRS>
 __global__ void __launch_bounds__(kGatherRowThreads) k_cell_gather_rows(CellGatherArgsT<P> a, int tr0, int fslot, int c0,
-                                                                        int c1, int ch) {
+                                                                        int c1, int ch, int pairs) {
     if (a.stop && *a.stop) return;
     extern __shared__ __align__(16) char rowsum[];
     __shared__ int2 walk[4 * kGatherRowThreads];  // per face: the warp's and the lane's next sublayer
-    gather_item_rows<NT, P, LdNC, U>(a, c0 + blockIdx.x * kGatherRowThreads + threadIdx.x, c1, tr0, fslot, ch,
+    unsigned b = blockIdx.x;
+    if constexpr (PAIRS) {
+        b = blockIdx.x / pairs;
+        const int g = NT * (int)(blockIdx.x - b * pairs);
+        tr0 += g;
+        fslot += g;
+    }
+    gather_item_rows<NT, P, LdNC, U>(a, c0 + b * kGatherRowThreads + threadIdx.x, c1, tr0, fslot, ch,
                                      rowsum + threadIdx.x * NT * sizeof(double), walk + threadIdx.x);
 }
 
@@ -332,7 +349,7 @@ cudaError_t launch_sweep(const SweepArgsT<P>& sw, cudaStream_t st, Band band) {
 }
 
 // The row gather's batch and largest chunk. A block is one warp; registers
-// (220 FP64, 168 mixed) admit 9 and 12 of them per SM, and the chunk's sums are
+// (164 FP64, 118 mixed) admit 12 and 17 of them per SM, and the chunk's sums are
 // sized to leave them an L1 that holds their rows in flight. Gather time at
 // 1440x1080x75 FP64, 2 tracers, batches of 8: chunks of 13 3.90 ms, 19 3.65,
 // 25 3.44, 38 (7 warps by shared memory) 4.53; batches of 4, 25 layers: 4.57;
@@ -347,15 +364,22 @@ struct RowGather {
 };
 
 template <int NT, class P>
-static void launch_gather_rows(const CellGatherArgsT<P>& cg, int tr, int slot, const BandRanges& r, cudaStream_t st) {
+static void launch_gather_rows(const CellGatherArgsT<P>& cg, int tr, int slot, const BandRanges& r, cudaStream_t st,
+                               int pairs = 1) {
     using G = RowGather<P>;
     const int chunks = (cg.nz + G::kChunk - 1) / G::kChunk, ch = (cg.nz + chunks - 1) / chunks;
     const size_t smem = (size_t)(ch + 2) * NT * plain::kGatherRowThreads * sizeof(double);
     const int c0 = r.j0 * cg.nx, c1 = r.j1 * cg.nx;
     launch_begin(K_CELL_UPDATE, st);
-    plain::k_cell_gather_rows<NT, P, G::kBatch>
-        <<<(unsigned)((c1 - c0 + plain::kGatherRowThreads - 1) / plain::kGatherRowThreads), plain::kGatherRowThreads,
-           smem, st>>>(cg, tr, slot, c0, c1, ch);
+    const unsigned nb = (unsigned)((c1 - c0 + plain::kGatherRowThreads - 1) / plain::kGatherRowThreads);
+    if (pairs > 1) {
+        if constexpr (NT == 2)
+            plain::k_cell_gather_rows<2, P, G::kBatch, true>
+                <<<nb * pairs, plain::kGatherRowThreads, smem, st>>>(cg, tr, slot, c0, c1, ch, pairs);
+    } else {
+        plain::k_cell_gather_rows<NT, P, G::kBatch, false>
+            <<<nb, plain::kGatherRowThreads, smem, st>>>(cg, tr, slot, c0, c1, ch, 1);
+    }
     launch_end(K_CELL_UPDATE, st);
 }
 
@@ -450,7 +474,7 @@ static void launch_gather_8(const CellGatherArgsT<P>& cg, int tr, const BandRang
 // ff.fslot0 .. ff.fslot0+NT-1.
 template <int NT, class P>
 static void launch_flux(const FaceFluxArgsT<P>& ff, int tr0, const BandRanges& r, const CellTuning& tune,
-                        cudaStream_t st) {
+                        cudaStream_t st, int pairs = 1) {
     const unsigned nb = face_blocks(r.f);
     if (nb == 0) return;
     const int kid = P::kMixed ? K_MIXED_FLUX : K_FACE_FLUX;
@@ -488,24 +512,34 @@ static void launch_flux(const FaceFluxArgsT<P>& ff, int tr0, const BandRanges& r
         }
     }
     launch_begin(kid, st);
-    plain::k_face_flux<NT, P><<<2 * nb, 128, 0, st>>>(ff, tr0, r.f);
+    if (pairs > 1) {
+        if constexpr (NT == 2) plain::k_face_flux<2, P, true><<<2 * nb * pairs, 128, 0, st>>>(ff, tr0, pairs, r.f);
+    } else {
+        plain::k_face_flux<NT, P, false><<<2 * nb, 128, 0, st>>>(ff, tr0, 1, r.f);
+    }
     launch_end(kid, st);
 }
 
 // The gathers of tracers tr0 .. tr0+NS-1, whose fluxes sit in slots 0 .. NS-1:
 // one launch of 8 tracers (WIDE: the fluxes of two face-flux launches), or
 // launches of 4 or 2 tracers, which read consecutive slots.
+// The row gathers of n tracers from tr0 on, whose fluxes sit in slots 0 .. n-1:
+// pairs, and an odd last tracer alone.
+template <class P>
+static void launch_row_gathers(const CellGatherArgsT<P>& cg, int tr0, int n, const BandRanges& r, cudaStream_t st) {
+    if (r.j1 <= r.j0) return;
+    if (n > 1) launch_gather_rows<2, P>(cg, tr0, 0, r, st, n / 2);
+    if (n & 1) launch_gather_rows<1, P>(cg, tr0 + n - 1, n - 1, r, st);
+}
+
 template <int NS, class P, bool WIDE = false>
 static void launch_gathers(const CellGatherArgsT<P>& cg, int tr0, const BandRanges& r, const CellTuning& tune,
                            cudaStream_t st) {
     const dim3 block(tune.bx, tune.by);
     const dim3 cgrid((cg.nx + tune.bx - 1) / tune.bx, (r.j1 - r.j0 + tune.by - 1) / tune.by);
     if (cgrid.y == 0) return;
-    if (tune.gather_rows) {  // pairs; an odd last tracer, or a flux buffer of one slot, alone
-        for (int g = 0; g < NS && tr0 + g < cg.ntr; g += 2) {
-            if (g + 1 < NS && tr0 + g + 1 < cg.ntr) launch_gather_rows<2, P>(cg, tr0 + g, g, r, st);
-            else launch_gather_rows<1, P>(cg, tr0 + g, g, r, st);
-        }
+    if (tune.gather_rows) {
+        launch_row_gathers<P>(cg, tr0, min(NS, cg.ntr - tr0), r, st);
         return;
     }
     if constexpr (WIDE) {
@@ -622,7 +656,7 @@ FoldShape fold_shape(int nz, int ntr) {
 
 template <class P>
 cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& ff, const CellGatherArgsT<P>& cg,
-                           cudaStream_t st, Band band, int recon_from, int flux_from, bool pairs_only) {
+                           cudaStream_t st, Band band, int recon_from, int flux_from, bool no_fold) {
     const BandRanges r = band_ranges(rc_all.nx, rc_all.ny, band);
     // the tracers still to reconstruct: rc_all's from recon_from on
     ReconArgsT<P> rc = rc_all;
@@ -633,7 +667,7 @@ cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& 
         rc.ti = rc_all.ti + (size_t)recon_from * ncol * (rc_all.nz + 1);
         rc.ppm = rc_all.ppm + (size_t)recon_from * ncol * rc_all.nz;
     }
-    const FoldShape fs = pairs_only ? FoldShape{0, 0} : fold_shape<P>(rc.nz, ff.ntr);
+    const FoldShape fs = no_fold ? FoldShape{0, 0} : fold_shape<P>(rc.nz, ff.ntr);
     if (fs.nt > 0) {
         if (r.c1 > r.c0 && rc.ntr > 0) {
             launch_recon<P>(rc, r, st);
@@ -668,13 +702,33 @@ cudaError_t launch_phase_b(const ReconArgsT<P>& rc_all, const FaceFluxArgsT<P>& 
     if (r.c1 > r.c0 && rc.ntr > 0) {
         launch_recon<P>(rc, r, st);
     }
+    if (ff.slots < 1) return cudaErrorInvalidValue;
     CellTuning tune = cell_tuning();
-    if (pairs_only) {
-        tune.group = min(tune.group, 2);
-        tune.gather_tracers = 2;
-    }
+    if (ff.slots < tune.group) tune.group = ff.slots >= 4 ? 4 : ff.slots >= 2 ? 2 : 1;
+    if (ff.slots < 8 && tune.gather_tracers > 4) tune.gather_tracers = 4;
     const int group = flux_group(ff.ntr, tune);
     if (flux_from == 2) launch_gathers<2, P>(cg, 0, r, tune, st);  // T and S: fluxes from the sweep, slots 0 and 1
+    if (pairs_share_launches(ff.ntr, tune)) {
+        const int most = min(kPairsPerLaunch, ff.slots / 2);
+        for (int tr0 = flux_from; tr0 < ff.ntr; tr0 += 2 * most) {
+            const int n = min(2 * most, ff.ntr - tr0);
+            // 361x275x51 FP64, 5 tracers: fluxes 1.22 ms a pair at a time, 0.97 side by
+            // side; 720x576x50 mixed, 32 tracers: 15.4 and 15.9 (24 bytes of
+            // coefficients instead of 32, and the added registers)
+            if constexpr (P::kMixed) {
+                FaceFluxArgsT<P> fp = ff;
+                for (int g = 0; g < n; g += 2) {
+                    fp.fslot0 = g;
+                    launch_flux<2, P>(fp, tr0 + g, r, tune, st);
+                }
+            } else {
+                launch_flux<2, P>(ff, tr0, r, tune, st, (n + 1) / 2);
+            }
+            // gathers: 0.71 and 0.66 ms, 9.47 and 8.41
+            launch_row_gathers<P>(cg, tr0, n, r, st);
+        }
+        return cudaGetLastError();
+    }
     if (gather_spans_two(ff.ntr, tune)) {
         // two face-flux launches of 4 tracers (slots 0-3 and 4-7), one gather of 8
         for (int tr0 = flux_from; tr0 < ff.ntr; tr0 += 8) {
