@@ -128,6 +128,9 @@ int run_phase_a(int nx, int ny, int nz, const redi::EosParams& eos, const double
     sw.nx = nx; sw.ny = ny; sw.nz = nz; sw.rho0 = eos.rho0;
     sw.wet_u = wet_u; sw.wet_v = wet_v; sw.ifc = cs.ifc; sw.pint = cs.pint;
     sw.u = u; sw.v = v;
+    cs.packed = sw.packed = redi::packed_state(redi::cell_tuning(), eos.variant);
+    sw.sv_t = eos.alpha_T / (eos.rho0 * eos.rho0);  // ocean_eos.F90:511-512
+    sw.sv_s = -eos.beta_S / (eos.rho0 * eos.rho0);
     e = redi::launch_column_state(cs, st, band);
     if (e == cudaSuccess) e = redi::launch_sweep<P>(sw, st, band);
     if (e != cudaSuccess) return cuda_fail(e, "phase A launch");

@@ -136,7 +136,8 @@ __device__ __forceinline__ bool column_needed(int col, int nx, int ny, WetU wet_
            (j >= 1 && wet_v(i + nx * j)) || (j + 1 <= ny - 1 && wet_v(i + nx * (j + 1)));
 }
 
-template <class LD>
+// LIN: packed (ColumnStateArgs::packed), as the sweep's packed ring takes it (SweepWin).
+template <class LD, bool LIN = false>
 __device__ __forceinline__ void column_state_item(const ColumnStateArgs& a, int col) {
     const int ncol = a.nx * a.ny;
     const int nz = a.nz;
@@ -170,14 +171,18 @@ __device__ __forceinline__ void column_state_item(const ColumnStateArgs& a, int 
     auto emit = [&](int t, const double (&e)[2], const double (&)[2], double h_t) {
         if (t >= 2) P = P + grho * h_layer_above;  // Pint(t) = Pint(t-1) + g*rho0*h(t-1)
         double rho_i, sv_t = dsv_dt, sv_s = dsv_ds;
-        if (linear)
+        if (LIN || linear)
             rho_i = eos.rho0 + eos.beta_S * (e[1] - eos.S_ref) - eos.alpha_T * (e[0] - eos.T_ref);
         else  // WRIGHT_97 / ROQUET_SPV at the interface pressure (ocean_redi.F90:649-650)
             eos::nonlinear_point(eos.variant, e[0], e[1], P, rho_i, sv_t, sv_s);
         double2* q = reinterpret_cast<double2*>(ifc + (size_t)(t - 1) * ncol);
         q[0] = make_double2(e[0], e[1]);
-        q[1] = make_double2(-(rho_i * rho_i) * sv_t, -(rho_i * rho_i) * sv_s);
-        pint[(size_t)(t - 1) * ncol] = P;
+        if constexpr (LIN) {
+            q[1] = make_double2(-(rho_i * rho_i), P);
+        } else {
+            q[1] = make_double2(-(rho_i * rho_i) * sv_t, -(rho_i * rho_i) * sv_s);
+            pint[(size_t)(t - 1) * ncol] = P;
+        }
         h_layer_above = h_t;
     };
     stream_edges<2, decltype(fetch), decltype(emit), kColumnAhead>(nz, fetch, emit);

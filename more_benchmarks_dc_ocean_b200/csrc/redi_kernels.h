@@ -91,6 +91,7 @@ struct ColumnStateArgs {
     // is wet is never read by the sweep, and is not computed
     const double* wet_u = nullptr;
     const double* wet_v = nullptr;
+    bool packed = false;        // 32 bytes an interface, no pint (a linear equation of state; see packed_state)
     const int* stop = nullptr;  // a launch does nothing once *stop != 0
 };
 
@@ -103,7 +104,8 @@ struct SweepArgsT {
     const IfcState* ifc;
     const double* pint;
     FaceOutT<P> u, v;
-    double sv_t = 0.0, sv_s = 0.0;  // packed column state: its derivatives over -(rho * rho)
+    bool packed = false;            // the column state is packed
+    double sv_t = 0.0, sv_s = 0.0;  // then: its derivatives over -(rho * rho)
     const int* stop = nullptr;
 };
 using SweepArgs = SweepArgsT<PlainPrec>;
@@ -310,6 +312,10 @@ cudaError_t launch_column_state(const ColumnStateArgs& cs, cudaStream_t st, Band
 // launches of their own, in the sweep, or in the sweep with the column state
 // packed (a linear equation of state).
 enum class StepForm { kSeparate, kFlux, kFluxPacked };
+// Whether the sweep's default form takes the packed column state: a linear
+// equation of state, whose derivatives are one value an interface times two
+// constants of the run.
+inline bool packed_state(const CellTuning& t, int eos_variant) { return t.sweep_form == 4 && eos_is_linear(eos_variant); }
 // The fluxes go into the sweep when the default forms of the sweep and the
 // face flux are in force, Phase B is not the fused fold, and the flux buffer
 // has a slot for each of the two.

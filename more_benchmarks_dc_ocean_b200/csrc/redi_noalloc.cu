@@ -152,6 +152,9 @@ int redi_b200_opt_launch_noalloc(const int* nx_, const int* ny_, const int* nz_,
     uint8_t* vdry = udry + nu;
     sw.u = redi::FaceOut{uPoL, uPoR, uKoL, uKoR, uhEff, udry};
     sw.v = redi::FaceOut{vPoL, vPoR, vKoL, vKoR, vhEff, vdry};
+    cs.packed = sw.packed = redi::packed_state(redi::cell_tuning(), eos.variant);
+    sw.sv_t = eos.alpha_T / (eos.rho0 * eos.rho0);
+    sw.sv_s = -eos.beta_S / (eos.rho0 * eos.rho0);
     if (e == cudaSuccess) e = redi::launch_column_state(cs, st);
     if (e == cudaSuccess) e = redi::launch_sweep<redi::PlainPrec>(sw, st);
     // Per-face diffusivities resolved into the caller's slots (redi_face_copy).

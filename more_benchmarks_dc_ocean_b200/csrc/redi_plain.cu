@@ -52,10 +52,11 @@ struct FaceRange {
     int lo[2], hi[2];
 };
 
+template <bool LIN>
 __global__ void __launch_bounds__(128) k_column_state(ColumnStateArgs a, int c0, int c1) {
     if (a.stop && *a.stop) return;
     const int col = c0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (col < c1) column_state_item<LdNC>(a, col);
+    if (col < c1) column_state_item<LdNC, LIN>(a, col);
 }
 
 template <class P, bool TI, bool LIN>
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(128) k_neutral_sweep(SweepArgsT<P> a, FaceRang
 // A block's faces are first sorted into dry ones (handled at once) and wet
 // ones, which are compacted onto the block's leading threads in face order, so
 // the sweeps of a block with land run in as few warps as its wet faces fill.
-template <class P, int NR>
+template <class P, int NR, bool LIN>
 __global__ void __launch_bounds__(kSweepWinThreads) k_neutral_sweep_w(SweepArgsT<P> a, FaceRange r) {
     if (a.stop && *a.stop) return;
     extern __shared__ __align__(16) unsigned char sweep_win[];
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(kSweepWinThreads) k_neutral_sweep_w(SweepArgsT
     const bool wet = t < r.hi[d] && sweep_face_dry<P, LdNC>(a, d, t);
     const int n = block_compact<kSweepWinThreads>(wet, t, list, warp_n);
     if ((int)threadIdx.x < n)
-        sweep_item_win<P, LdNC, NR, true>(a, d, list[threadIdx.x], *reinterpret_cast<SweepWin<NR>*>(sweep_win));
+        sweep_item_win<P, LdNC, NR, true, LIN>(a, d, list[threadIdx.x], *reinterpret_cast<SweepWin<NR, LIN>*>(sweep_win));
 }
 
 // The same sweep with the fluxes of T and S evaluated as its surfaces are
@@ -282,7 +283,9 @@ cudaError_t launch_column_state(const ColumnStateArgs& cs, cudaStream_t st, Band
     const BandRanges r = band_ranges(cs.nx, cs.ny, band);
     if (r.c1 > r.c0) {
         launch_begin(K_COLUMN_STATE, st);
-        plain::k_column_state<<<(r.c1 - r.c0 + 127) / 128, 128, 0, st>>>(cs, r.c0, r.c1);
+        const unsigned nb = (unsigned)((r.c1 - r.c0 + 127) / 128);
+        if (cs.packed) plain::k_column_state<true><<<nb, 128, 0, st>>>(cs, r.c0, r.c1);
+        else plain::k_column_state<false><<<nb, 128, 0, st>>>(cs, r.c0, r.c1);
         launch_end(K_COLUMN_STATE, st);
     }
     return cudaGetLastError();
@@ -316,14 +319,14 @@ cudaError_t launch_eos_points(const EosParams& e, int n, const double* T, const 
     return cudaGetLastError();
 }
 
-template <class P, int NR>
+template <class P, int NR, bool LIN = false>
 static cudaError_t launch_sweep_w(const SweepArgsT<P>& sw, const plain::FaceRange& f, unsigned nb, cudaStream_t st) {
-    const size_t smem = sizeof(plain::SweepWin<NR>);
+    const size_t smem = sizeof(plain::SweepWin<NR, LIN>);
     cudaError_t e =
-        cudaFuncSetAttribute(plain::k_neutral_sweep_w<P, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(plain::k_neutral_sweep_w<P, NR, LIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const unsigned nbw = (unsigned)(((size_t)nb * 128 + plain::kSweepWinThreads - 1) / plain::kSweepWinThreads);
-    plain::k_neutral_sweep_w<P, NR><<<2 * nbw, plain::kSweepWinThreads, smem, st>>>(sw, f);
+    plain::k_neutral_sweep_w<P, NR, LIN><<<2 * nbw, plain::kSweepWinThreads, smem, st>>>(sw, f);
     return cudaSuccess;
 }
 
@@ -334,10 +337,11 @@ cudaError_t launch_sweep(const SweepArgsT<P>& sw, cudaStream_t st, Band band) {
     if (nb > 0) {
         const int kid = P::kMixed ? K_MIXED_SWEEP : K_NEUTRAL_SWEEP;
         const int form = cell_tuning().sweep_form;
+        if (sw.packed && form != 4) return cudaErrorInvalidValue;  // only that form reads it
         launch_begin(kid, st);
         if (form >= 3 && form <= 5) {
             cudaError_t e = form == 3   ? launch_sweep_w<P, 3>(sw, r.f, nb, st)
-                            : form == 4 ? launch_sweep_w<P, 4>(sw, r.f, nb, st)
+                            : form == 4 ? (sw.packed ? launch_sweep_w<P, 4, true>(sw, r.f, nb, st) : launch_sweep_w<P, 4>(sw, r.f, nb, st))
                                         : launch_sweep_w<P, 5>(sw, r.f, nb, st);
             if (e != cudaSuccess) return e;
         } else {
