@@ -469,7 +469,8 @@ def run_b200(args, rank, world, local_rank):
             "gpu_launches": int(n1 - n0),
             "tuning": {"cell_update_tile": list(tuning["best"][:2]), "vertical_chunk": tuning["best"][2],
                        "gather_sums": {0: "registers", 1: "shared memory", 2: "shared memory, 8-deep batches",
-                                       3: "shared memory, pipelined batches of 4"}[
+                                       3: "shared memory, pipelined batches of 4",
+                                       4: "shared memory, a warp on whole rows"}[
                            tuning["best"][3] if len(tuning["best"]) > 3 else 0],
                        "tracer_group": tuning.get("tracer_group"),
                        "candidates_ms": tuning["ms"]} if tuning else None,
