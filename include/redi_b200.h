@@ -424,10 +424,12 @@ REDI_B200_API int redi_b200_batch_get_tuning(const redi_b200_batch* b, int* tile
                                              int* occupancy, int* grid);
 
 /* Form of the step: one persistent kernel over the whole work queue, or the
- * handle API's launches for every domain on a few streams (the default); both
- * are captured in the graph. Results do not depend on it. The accounting below
- * is the persistent kernel's: a step with it on takes that form, and the launch
- * shape above is that kernel's. get returns the form in force. */
+ * handle API's launches for every domain on a few streams; both are captured in
+ * the graph. Results do not depend on it. AUTO (the default) takes the launches
+ * unless a domain is held. The accounting below is the persistent kernel's: a
+ * step with it on takes that form, and the launch shape above is that kernel's.
+ * get returns the form of the next step (PERSISTENT or LAUNCHES). */
+#define REDI_B200_BATCH_AUTO 0
 #define REDI_B200_BATCH_PERSISTENT 1
 #define REDI_B200_BATCH_LAUNCHES 2
 REDI_B200_API int redi_b200_batch_set_form(redi_b200_batch* b, int form);

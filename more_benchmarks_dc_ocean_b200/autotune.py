@@ -325,6 +325,8 @@ def tune_batch(batch, candidates: Optional[Iterable[Tuple[int, int, int]]] = Non
     batch.set_form(R.BATCH_LAUNCHES)
     t = timed()
     ms["launches"] = round(t, 4)
-    if t > times[best]:
-        batch.set_form(R.BATCH_PERSISTENT)
+    faster = R.BATCH_LAUNCHES if t <= times[best] else R.BATCH_PERSISTENT
+    batch.set_form(R.BATCH_AUTO)
+    if batch.get_form() != faster:  # only where the batch's own choice is the slower one is it overruled
+        batch.set_form(faster)
     return {"best": best, "form": batch.get_form(), "ms": ms}

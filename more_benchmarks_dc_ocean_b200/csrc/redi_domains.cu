@@ -130,8 +130,9 @@ __device__ __forceinline__ bool wait_released(const int* held, int* status, unsi
 }
 
 // The start of a step made of launches per domain: the control block cleared,
-// then a bounded wait for held domains; on expiry the status makes every
-// launch that follows do nothing (their `stop` word).
+// then a bounded wait for held domains (a form set by the caller, or a hold that
+// came after the step was enqueued); on expiry the status makes every launch
+// that follows do nothing (their `stop` word).
 __global__ void __launch_bounds__(kThreads) k_batch_gate(const int* held, int ndomains, Control* ctl,
                                                          unsigned long long limit_ns) {
     for (int x = threadIdx.x; x < (int)(sizeof(Control) / sizeof(int)); x += kThreads) reinterpret_cast<int*>(ctl)[x] = 0;
@@ -246,7 +247,10 @@ struct redi_b200_batch {
     int use_graph = 1;
     int occ = 4;       // register budget: blocks per SM (4, 5 or 6)
     int account = 0;   // per-stage time accounting in the kernel
-    int form = REDI_B200_BATCH_LAUNCHES;
+    int form = REDI_B200_BATCH_AUTO;
+    std::vector<unsigned char> held;  // host copy of d_held
+    int nheld = 0;
+    bool exec_launches = false;       // the form that `exec` holds
     std::vector<cudaStream_t> lanes;  // launches per domain: the streams they run on
     std::vector<cudaEvent_t> lane_done;
     cudaEvent_t fork = nullptr;
@@ -504,6 +508,7 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
     if (e == cudaSuccess) b->allocs.push_back(b->d_held);
     if (e != cudaSuccess) return bfail(REDI_B200_E_NOMEM, std::string("redi_b200_batch_create: ") + cudaGetErrorString(e));
     cudaMemset(b->d_held, 0, sizeof(int) * n);
+    b->held.assign(n, 0);
     cudaMemset(b->d_ctl, 0, sizeof(Control));
     const int rc = layout<P>(b);
     if (rc < 0) return rc;
@@ -594,8 +599,13 @@ cudaError_t enqueue_launches(redi_b200_batch* b, cudaStream_t st) {
     return e;
 }
 
+// The form of the next step. The accounting is the persistent kernel's. Left to
+// itself, a step with a held domain takes it too: there a domain waits tile by
+// tile and the others go on, where the launches' gate stops all of them.
 bool by_launches(const redi_b200_batch* b) {
-    return b->form == REDI_B200_BATCH_LAUNCHES && !b->account;  // the accounting is the persistent kernel's
+    if (b->account) return false;
+    if (b->form == REDI_B200_BATCH_AUTO) return b->nheld == 0;
+    return b->form == REDI_B200_BATCH_LAUNCHES;
 }
 
 cudaError_t enqueue_any(redi_b200_batch* b, cudaStream_t st, bool instrument) {
@@ -660,8 +670,10 @@ int redi_b200_batch_step(redi_b200_batch* b, void* stream) {
         cudaError_t e = enqueue_any(b, st, true);
         return e == cudaSuccess ? REDI_B200_OK : bfail(REDI_B200_E_CUDA, cudaGetErrorString(e));
     }
+    const bool launches = by_launches(b);
+    if (b->exec && b->exec_launches != launches) drop_graph(b);
     if (!b->exec) {
-        // Capture the step (counter reset + persistent kernel) once on a private stream.
+        // Capture the step once on a private stream.
         cudaStream_t cap;
         cudaError_t e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
@@ -673,6 +685,7 @@ int redi_b200_batch_step(redi_b200_batch* b, void* stream) {
         if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec, b->graph, 0);
         cudaStreamDestroy(cap);
         if (e != cudaSuccess) return bfail(REDI_B200_E_CUDA, std::string("redi_b200_batch_step: graph: ") + cudaGetErrorString(e));
+        b->exec_launches = launches;
     }
     redi::launch_begin(redi::K_DOMAIN_PERSISTENT, st);
     cudaError_t e = cudaGraphLaunch(b->exec, st);
@@ -730,10 +743,9 @@ int redi_b200_batch_get_tuning(const redi_b200_batch* b, int* tile_bx, int* tile
 
 int redi_b200_batch_set_form(redi_b200_batch* b, int form) {
     if (!b) return bfail(REDI_B200_E_ARG, "redi_b200_batch_set_form: NULL batch");
-    if (form != REDI_B200_BATCH_PERSISTENT && form != REDI_B200_BATCH_LAUNCHES)
-        return bfail(REDI_B200_E_ARG, "redi_b200_batch_set_form: form must be 1 or 2");
-    if (form != b->form) drop_graph(b);
-    b->form = form;
+    if (form != REDI_B200_BATCH_AUTO && form != REDI_B200_BATCH_PERSISTENT && form != REDI_B200_BATCH_LAUNCHES)
+        return bfail(REDI_B200_E_ARG, "redi_b200_batch_set_form: form must be 0, 1 or 2");
+    b->form = form;  // the next step drops a graph of the other form
     return REDI_B200_OK;
 }
 
@@ -766,7 +778,10 @@ int redi_b200_batch_hold(redi_b200_batch* b, int domain, int hold) {
     if (!b || domain < 0 || domain >= b->ndomains) return bfail(REDI_B200_E_ARG, "redi_b200_batch_hold: bad domain");
     const int v = hold != 0;
     cudaError_t e = cudaMemcpy(b->d_held + domain, &v, sizeof(int), cudaMemcpyHostToDevice);
-    return e == cudaSuccess ? REDI_B200_OK : bfail(REDI_B200_E_CUDA, cudaGetErrorString(e));
+    if (e != cudaSuccess) return bfail(REDI_B200_E_CUDA, cudaGetErrorString(e));
+    b->nheld += v - b->held[domain];
+    b->held[domain] = (unsigned char)v;
+    return REDI_B200_OK;
 }
 
 long long redi_b200_batch_updates(const redi_b200_batch* b) {

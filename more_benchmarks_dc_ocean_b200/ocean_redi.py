@@ -486,7 +486,7 @@ def step(dp: DeviceProblem, redi: OceanRedi, nsteps: int = 1, stream=None) -> No
 # Many domains in one persistent launch (no counterpart in the reference)
 # ---------------------------------------------------------------------------
 STATUS_TIMEOUT = 1
-BATCH_PERSISTENT, BATCH_LAUNCHES = 1, 2
+BATCH_AUTO, BATCH_PERSISTENT, BATCH_LAUNCHES = 0, 1, 2
 STAGE_NAMES = ("column_state", "neutral_sweep", "tracer_recon")
 
 
@@ -590,12 +590,13 @@ class RediBatch:
         return {"tile": (bx.value, by.value), "chunk": ch.value, "occupancy": occ.value, "grid": grid.value}
 
     def set_form(self, form: int) -> None:
-        """BATCH_PERSISTENT (one kernel over the work queue) or BATCH_LAUNCHES (every domain's launches
-        on a few streams, the default); results do not depend on it."""
+        """BATCH_PERSISTENT (one kernel over the work queue), BATCH_LAUNCHES (every domain's launches on a
+        few streams) or BATCH_AUTO (the default: the launches, unless a domain is held); results do not
+        depend on it."""
         _check(_batch_lib().redi_b200_batch_set_form(self._h, int(form)))
 
     def get_form(self) -> int:
-        """The form a step takes now: BATCH_PERSISTENT or BATCH_LAUNCHES."""
+        """The form the next step takes: BATCH_PERSISTENT or BATCH_LAUNCHES."""
         return _check(_batch_lib().redi_b200_batch_get_form(self._h))
 
     def set_accounting(self, on: bool = True) -> None:

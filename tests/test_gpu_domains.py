@@ -203,3 +203,31 @@ def test_batch_launches_time_out_on_a_held_domain(redi_lib):
         ref = _handle_run(R, p, 1)
         for n, (a, c) in enumerate(zip(g, ref)):
             _assert_exact(f"{p.name} tracer {n}", a, c)
+
+
+def test_batch_goes_on_around_a_held_domain(redi_lib):
+    """Left to itself, a step with a held domain names it in the status and advances every other domain by
+    one step; the held one is untouched, and a form that the caller chose stays in force."""
+    R = redi_lib
+    ps = _domains()
+    dps = [R.to_device(p) for p in ps]
+    b = R.RediBatch(dps)
+    assert b.get_form() == R.BATCH_LAUNCHES
+    b.set_wait_limit(100_000_000)  # 100 ms: the other domains take a fraction of one
+    b.hold(2)
+    assert b.get_form() == R.BATCH_PERSISTENT
+    b.step()
+    st = b.status()
+    assert st["status"] == R.STATUS_TIMEOUT and st["domain"] == 2 and st["stage"] in (0, 1), st
+    for k, (p, dp) in enumerate(zip(ps, dps)):
+        ref = p.tracers if k == 2 else _handle_run(R, p, 1)
+        for n, (t, c) in enumerate(zip(dp.ms.tracers, ref)):
+            _assert_exact(f"{p.name} tracer {n}", t.cpu().numpy(), c)
+    b.hold(2, False)
+    assert b.get_form() == R.BATCH_LAUNCHES
+    b.step()
+    assert b.status()["status"] == 0
+    b.set_form(R.BATCH_LAUNCHES)
+    b.hold(2)
+    assert b.get_form() == R.BATCH_LAUNCHES
+    b.destroy()
