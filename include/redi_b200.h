@@ -425,8 +425,9 @@ REDI_B200_API int redi_b200_batch_get_tuning(const redi_b200_batch* b, int* tile
 
 /* Form of the step: one persistent kernel over the whole work queue, or the
  * handle API's launches for every domain on a few streams; both are captured in
- * the graph. Results do not depend on it. AUTO (the default) takes the launches
- * unless a domain is held. The accounting below is the persistent kernel's: a
+ * the graph. Results do not depend on it. AUTO (the default) takes the launches,
+ * but the persistent kernel for many small domains (whose launches would take
+ * longer to start than to run) and while a domain is held. The accounting below is the persistent kernel's: a
  * step with it on takes that form, and the launch shape above is that kernel's.
  * get returns the form of the next step (PERSISTENT or LAUNCHES). */
 #define REDI_B200_BATCH_AUTO 0

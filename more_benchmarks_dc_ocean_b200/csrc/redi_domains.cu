@@ -1,17 +1,17 @@
 // Many independent regional domains of uneven size, in one of two forms.
 //
-// Launches per domain (the default): a domain's step is the handle API's own
-// launches on one of a few streams, all of it one graph. The stages then have
-// the registers, the shared memory and the L1 of kernels of their own, where
-// the persistent kernel's stages share one budget and read what they made
-// through L2 only. Measured against the persistent kernel: 12 domains of up to
-// 512x512x75 with 6 tracers 14.5 ms instead of 29.6, 64 of 64x64x50 8.7 instead
-// of 18.7, 12 of 16x16x8 with 2 tracers 0.095 instead of 0.159; nowhere slower.
+// Launches per domain: a domain's step is the handle API's own launches on one
+// of a few streams, all of it one graph. The stages then have the registers, the
+// shared memory and the L1 of kernels of their own, where the persistent
+// kernel's stages share one budget and read what they made through L2 only: 12
+// domains of up to 512x512x75 with 6 tracers take 14.3 ms instead of 29.6.
 //
-// The persistent kernel (its per-stage accounting, and on request): a step of every domain (Phase A then Phase B, all tracers) is cut into work
-// items: tiles of columns (interface state, tracer reconstruction), tiles of
-// faces (neutral sweep, face fluxes of one tracer pair) and 2-D tiles of cells
-// (the ordered gather of one tracer pair). The host builds the item queue once:
+// The persistent kernel (many small domains, whose launches take longer to start
+// than to run, see prefer_persistent; a step with a held domain; its per-stage
+// accounting; on request): a step of every domain (Phase A then Phase B, all
+// tracers) is cut into work items: tiles of columns (interface state, tracer
+// reconstruction), tiles of faces (neutral sweep, face fluxes of one tracer
+// pair) and 2-D tiles of cells (the ordered gather of one tracer pair). The host builds the item queue once:
 // stage by stage, and within a stage domain by domain, largest domain first
 // (longest-processing-time order), so an item's predecessors always sit earlier
 // in the queue. One persistent grid (as many blocks as fit on the GPU at once)
@@ -248,6 +248,7 @@ struct redi_b200_batch {
     int occ = 4;       // register budget: blocks per SM (4, 5 or 6)
     int account = 0;   // per-stage time accounting in the kernel
     int form = REDI_B200_BATCH_AUTO;
+    bool many_small = false;          // the persistent kernel is the faster form (prefer_persistent)
     std::vector<unsigned char> held;  // host copy of d_held
     int nheld = 0;
     bool exec_launches = false;       // the form that `exec` holds
@@ -387,6 +388,29 @@ int layout_any(redi_b200_batch* b) {
 // 12 of them, 12 of up to 512x512x75 14.9 / 14.6 / 14.7 / 14.4.
 constexpr int kLanes = 12;
 
+// Launches of one domain's step: columns, sweep, gather; with passive tracers
+// their reconstruction, and fluxes (mixed precision: a pair at a time) and
+// gathers a few pairs at a time.
+template <class P>
+int step_nodes(int ntr) {
+    const int pairs = (ntr - 1) / 2, groups = (pairs + redi::kPairsPerLaunch - 1) / redi::kPairsPerLaunch;
+    return 3 + (pairs ? 1 + (P::kMixed ? pairs : groups) + groups : 0);
+}
+
+// Whether the persistent kernel steps the batch faster than the launches. A graph
+// starts its nodes one after another, 1.4 us apart however small they are, and
+// their work adds 0.045 ns a unit of `cost`; the persistent kernel takes 0.06 ms
+// and 0.052 ms a tracer pair for its chain of stages, and 0.125 ns a unit. FP64,
+// T and S, persistent and launches in ms: 12 domains of 16x16x8 0.135 and 0.052, 32
+// 0.165 and 0.140, 64 0.157 and 0.282, 1000 1.46 and 4.22; 1000 of 6x6x4 0.33 and
+// 2.88; 400 of 20x20x12 1.63 and 2.25; 200 of 24x24x15 1.32 and 1.30; 400 of 32x32x10
+// 2.71 and 2.10; 1000 of 32x32x20 13.2 and 8.8; 250 of 64x64x25 12.7 and 4.5. With 6
+// tracers 20 of 16x16x8 0.31 and 0.17, 100 0.41 and 0.87. Mixed precision is within a
+// tenth of these on both sides.
+bool prefer_persistent(int nodes, int pairs, double cost) {
+    return 1400.0 * nodes > 6.0e4 + 5.2e4 * pairs + 0.08 * cost;
+}
+
 template <class P>
 int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
     using Ko = typename P::Ko;
@@ -394,6 +418,7 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
     b->host_doms.assign(sizeof(DomainDev<P>) * n, 0);
     DomainDev<P>* hd = reinterpret_cast<DomainDev<P>*>(b->host_doms.data());
     b->cost.assign(n, 0.0);
+    int nodes = 1, most_pairs = 1;  // of the launches' graph: the gate, and every domain's
     cudaError_t e0 = cudaMalloc((void**)&b->d_ctl, sizeof(Control));
     if (e0 != cudaSuccess) return bfail(REDI_B200_E_NOMEM, std::string("redi_b200_batch_create: ") + cudaGetErrorString(e0));
     b->allocs.push_back(b->d_ctl);
@@ -500,6 +525,8 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
         d.ntiles[redi::domains::S_RECON] = (int)((ncol * npairs + kThreads - 1) / kThreads);
         for (int g = 0; g < npairs; ++g) d.ntiles[redi::domains::S_PAIR0 + 2 * g] = face_tiles;
         b->cost[k] = (double)ncol * nz * (2.0 + ntr);
+        nodes += step_nodes<P>(ntr);
+        most_pairs = std::max(most_pairs, npairs);
         b->updates.push_back((long long)D.grid.nx_phys * D.grid.ny_phys * nz * ntr);
     }
     cudaError_t e = cudaMalloc(&b->d_doms, sizeof(DomainDev<P>) * n);
@@ -512,6 +539,7 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
     cudaMemset(b->d_ctl, 0, sizeof(Control));
     const int rc = layout<P>(b);
     if (rc < 0) return rc;
+    b->many_small = prefer_persistent(nodes, most_pairs, std::accumulate(b->cost.begin(), b->cost.end(), 0.0));
     // The launches per domain run on a few streams, each domain on the one with
     // the least work so far (a stream's launches follow one another; other
     // streams' launches fill the ends of its grids).
@@ -604,7 +632,7 @@ cudaError_t enqueue_launches(redi_b200_batch* b, cudaStream_t st) {
 // tile and the others go on, where the launches' gate stops all of them.
 bool by_launches(const redi_b200_batch* b) {
     if (b->account) return false;
-    if (b->form == REDI_B200_BATCH_AUTO) return b->nheld == 0;
+    if (b->form == REDI_B200_BATCH_AUTO) return b->nheld == 0 && !b->many_small;
     return b->form == REDI_B200_BATCH_LAUNCHES;
 }
 

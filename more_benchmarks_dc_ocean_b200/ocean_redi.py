@@ -591,8 +591,8 @@ class RediBatch:
 
     def set_form(self, form: int) -> None:
         """BATCH_PERSISTENT (one kernel over the work queue), BATCH_LAUNCHES (every domain's launches on a
-        few streams) or BATCH_AUTO (the default: the launches, unless a domain is held); results do not
-        depend on it."""
+        few streams) or BATCH_AUTO (the default: the launches, but one kernel for many small domains and
+        while a domain is held); results do not depend on it."""
         _check(_batch_lib().redi_b200_batch_set_form(self._h, int(form)))
 
     def get_form(self) -> int:

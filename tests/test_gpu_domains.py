@@ -231,3 +231,26 @@ def test_batch_goes_on_around_a_held_domain(redi_lib):
     b.hold(2)
     assert b.get_form() == R.BATCH_LAUNCHES
     b.destroy()
+
+
+@pytest.mark.parametrize("n,shape,npas,launches", [(12, (16, 16, 8), 0, True), (200, (16, 16, 8), 0, False),
+                                                   (200, (10, 9, 5), 3, False), (1, (6, 6, 1), 0, True)])
+def test_batch_form_by_size(redi_lib, n, shape, npas, launches):
+    """Left to itself, a batch of many small domains takes one kernel, others the launches; the step is the
+    other form's bit for bit."""
+    R = redi_lib
+    ps = [inputs.make_problem(*shape, n_seamounts=3, land_fraction=0.2, n_passive=npas, seed=50 + k) for k in range(3)]
+    out = []
+    for form in (R.BATCH_AUTO, R.BATCH_PERSISTENT if launches else R.BATCH_LAUNCHES):
+        dps = [R.to_device(ps[k % 3]) for k in range(n)]
+        b = R.RediBatch(dps)
+        b.set_form(form)
+        assert (b.get_form() == R.BATCH_LAUNCHES) == (launches == (form == R.BATCH_AUTO))
+        b.step(2)
+        st = b.status()
+        b.destroy()
+        assert st["status"] == 0 and st["bad"] == 0, st
+        out.append([[t.cpu().numpy() for t in dp.ms.tracers] for dp in dps])
+    for k, (x, y) in enumerate(zip(*out)):
+        for i, (a, c) in enumerate(zip(x, y)):
+            _assert_exact(f"domain {k} tracer {i}", a, c)
