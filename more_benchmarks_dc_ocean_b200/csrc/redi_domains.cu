@@ -67,7 +67,6 @@ struct DomainDev {
     int ntiles[kMaxStages];
     int nu_tiles;   // face stages: tiles < nu_tiles are u-faces
     int gx;         // gather tiles along x
-    int ts_first;   // tracers 0 and 1 are T and S (1), S and T (2) or others (0)
 };
 
 struct Item {
@@ -240,6 +239,17 @@ using redi::domains::Item;
 using redi::domains::kMaxStages;
 using redi::domains::kThreads;
 
+// Where a domain's launches keep their buffers when the sweep evaluates the fluxes
+// of T and S. Its scratch is laid out twice: until those two are gathered it holds
+// Phase A's state, their limited layers and their fluxes; after that the passive
+// tracers' reconstruction and as many slots of fluxes as the same bytes take.
+struct LaunchLayout {
+    char* scratch;
+    size_t ppm_ts, flux_ts;  // offsets, T and S
+    int slots;               // flux slots of the passive tracers
+    int ts_first;            // tracers 0 and 1 are T and S (1) or S and T (2); 0: Phase A and Phase B in turn
+};
+
 struct redi_b200_batch {
     int precision = REDI_B200_FP64;
     int ndomains = 0;
@@ -257,6 +267,7 @@ struct redi_b200_batch {
     cudaEvent_t fork = nullptr;
     std::vector<int> lane_of;      // domain -> lane
     std::vector<int> order;        // domains in decreasing cost
+    std::vector<LaunchLayout> layouts;
     unsigned long long tally[redi::K_NUM] = {};  // the captured step's launches
     int grid = 0;
     int nitems = 0;
@@ -390,10 +401,10 @@ constexpr int kLanes = 12;
 
 // Launches of one domain's step: columns, sweep, gather; with passive tracers
 // their reconstruction, and fluxes (mixed precision: a pair at a time) and
-// gathers a few pairs at a time.
+// gathers of `at_once` pairs.
 template <class P>
-int step_nodes(int ntr) {
-    const int pairs = (ntr - 1) / 2, groups = (pairs + redi::kPairsPerLaunch - 1) / redi::kPairsPerLaunch;
+int step_nodes(int ntr, int at_once) {
+    const int pairs = (ntr - 1) / 2, groups = pairs ? (pairs + at_once - 1) / at_once : 0;
     return 3 + (pairs ? 1 + (P::kMixed ? pairs : groups) + groups : 0);
 }
 
@@ -450,13 +461,30 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
                               up256(nv * ns * sizeof(Ko)) * 2 + up256(nu * (ns - 1) * sizeof(He)) +
                               up256(nv * (ns - 1) * sizeof(He)) + up256(nu) + up256(nv);
         const size_t a_b = redi::phase_a_scratch(nx, ny, nz);
-        const int slots = 2 * std::min(redi::kPairsPerLaunch, (ntr + 1) / 2);
-        const size_t rb = redi::recon_bytes<P>(nx, ny, nz, ntr), fb = redi::flux_bytes<P>(nx, ny, nz, slots);
-        // Phase A's state beside Phase B's buffers: the sweep that evaluates the fluxes needs both
-        const size_t scratch = up256(rb) + up256(fb) + a_b;
+        const size_t rb = redi::recon_bytes<P>(nx, ny, nz, ntr), fb = redi::flux_bytes<P>(nx, ny, nz, 2);
+        // What the two phases need in turn (Phase A's state shares the bytes of Phase B's buffers), and with the
+        // fluxes of T and S inside the sweep, where both live at a time: more only for two tracers, by 6 to 9 %
+        // of all that the domain takes. Without room for that the phases run in turn.
+        const size_t in_turn = std::max(a_b, up256(rb) + fb);
+        LaunchLayout lay{};
+        lay.ts_first = D.ms.idx_temperature == 1 && D.ms.idx_salinity == 2   ? 1
+                       : D.ms.idx_temperature == 2 && D.ms.idx_salinity == 1 ? 2
+                                                                             : 0;
+        lay.ppm_ts = up256(redi::eos_is_linear(D.eos.variant) ? ncol * (nz + 1) * sizeof(redi::IfcState) : a_b);
+        lay.flux_ts = up256(lay.ppm_ts + 2 * ncol * nz * sizeof(typename P::Ppm));
+        size_t scratch = lay.ts_first ? std::max(in_turn, lay.flux_ts + fb) : in_turn;
         char* base = nullptr;
         cudaError_t e = cudaMalloc((void**)&base, coef_b + up256(scratch));
+        if (e == cudaErrorMemoryAllocation && scratch > in_turn) {
+            cudaGetLastError();
+            lay.ts_first = 0;
+            scratch = in_turn;
+            e = cudaMalloc((void**)&base, coef_b + up256(scratch));
+        }
         if (e != cudaSuccess) return bfail(REDI_B200_E_NOMEM, std::string("redi_b200_batch_create: ") + cudaGetErrorString(e));
+        const size_t rest = ntr > 2 ? up256(redi::recon_bytes<P>(nx, ny, nz, ntr - 2)) : 0;
+        lay.slots = 2 * std::min(redi::kPairsPerLaunch, (ntr - 1) / 2);
+        while (lay.slots > 2 && rest + redi::flux_bytes<P>(nx, ny, nz, lay.slots) > scratch) lay.slots -= 2;
         b->allocs.push_back(base);
         cudaMemset(base, 0, coef_b);
         char* q = base;
@@ -470,13 +498,15 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
         v.dry = (uint8_t*)take(nv);
         u.keep = v.keep = true;
         char* sc = base + coef_b;
+        lay.scratch = sc;
+        b->layouts.push_back(lay);
         DomainDev<P>& d = hd[k];
         std::memset(&d, 0, sizeof(d));
         const double* th = D.ms.hTr[D.ms.idx_temperature - 1];
         const double* sh = D.ms.hTr[D.ms.idx_salinity - 1];
         d.cs = redi::ColumnStateArgs{nx, ny, nz, redi::EosParams{D.eos.variant, D.eos.rho0, D.eos.T_ref, D.eos.S_ref,
                                                                   D.eos.alpha_T, D.eos.beta_S},
-                                     D.ms.h_layer, th, sh, (redi::IfcState*)(sc + up256(rb) + up256(fb)), nullptr};
+                                     D.ms.h_layer, th, sh, (redi::IfcState*)sc, nullptr};
         d.cs.pint = (double*)(d.cs.ifc + ncol * (nz + 1));
         d.cs.wet_u = D.metrics.wet_u; d.cs.wet_v = D.metrics.wet_v;
         d.sw.nx = nx; d.sw.ny = ny; d.sw.nz = nz; d.sw.rho0 = D.eos.rho0;
@@ -484,9 +514,6 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
         d.sw.u = u; d.sw.v = v;
         d.sw.sv_t = D.eos.alpha_T / (D.eos.rho0 * D.eos.rho0);
         d.sw.sv_s = -D.eos.beta_S / (D.eos.rho0 * D.eos.rho0);
-        d.ts_first = D.ms.idx_temperature == 1 && D.ms.idx_salinity == 2   ? 1
-                     : D.ms.idx_temperature == 2 && D.ms.idx_salinity == 1 ? 2
-                                                                           : 0;
         d.cs.stop = d.sw.stop = d.rc.stop = d.ff.stop = d.cg.stop = &b->d_ctl->status;
         d.rc.nx = nx; d.rc.ny = ny; d.rc.nz = nz; d.rc.ntr = ntr; d.rc.h = D.ms.h_layer;
         d.rc.ti = (double*)sc;
@@ -504,8 +531,8 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
         ff.v = redi::FaceInT<P>{v.PoL, v.PoR, v.KoL, v.KoR, v.hEff, v.dry};
         ff.ti = d.rc.ti; ff.ppm = d.rc.ppm;
         ff.Fu = (typename P::Flux*)(sc + up256(rb));
-        ff.slots = slots;
-        ff.Fv = ff.Fu + (size_t)slots * (2 * nz + 1) * nu;
+        ff.slots = 2;
+        ff.Fv = ff.Fu + (size_t)2 * (2 * nz + 1) * nu;
         auto& cg = d.cg;
         cg.nx = nx; cg.ny = ny; cg.nz = nz; cg.ntr = ntr; cg.nghost = ff.nghost; cg.nxp = ff.nxp; cg.nyp = ff.nyp;
         cg.wall_w = walls[0]; cg.wall_e = walls[1]; cg.wall_s = walls[2]; cg.wall_n = walls[3];
@@ -525,7 +552,7 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
         d.ntiles[redi::domains::S_RECON] = (int)((ncol * npairs + kThreads - 1) / kThreads);
         for (int g = 0; g < npairs; ++g) d.ntiles[redi::domains::S_PAIR0 + 2 * g] = face_tiles;
         b->cost[k] = (double)ncol * nz * (2.0 + ntr);
-        nodes += step_nodes<P>(ntr);
+        nodes += step_nodes<P>(ntr, lay.slots / 2);
         most_pairs = std::max(most_pairs, npairs);
         b->updates.push_back((long long)D.grid.nx_phys * D.grid.ny_phys * nz * ntr);
     }
@@ -588,25 +615,56 @@ void count_tally(const redi_b200_batch* b) {
         if (b->tally[k]) redi::count_launches(k, b->tally[k]);
 }
 
+// The flux buffer at `at`, with room for the fluxes of `slots` tracers, as tracers [t0, t0 + n) use it.
+template <class P>
+void flux_buffer(redi::FaceFluxArgsT<P>& ff, redi::CellGatherArgsT<P>& cg, char* at, int slots, int t0, int n) {
+    ff.ntr = cg.ntr = n;
+    ff.slots = slots;
+    ff.Fu = reinterpret_cast<typename P::Flux*>(at);
+    ff.Fv = ff.Fu + (size_t)slots * (2 * ff.nz + 1) * (size_t)(ff.nx + 1) * ff.ny;
+    cg.Fu = ff.Fu;
+    cg.Fv = ff.Fv;
+    for (int k = 0; k < n; ++k) {
+        cg.htr[k] = cg.htr[t0 + k];
+        cg.htr_in[k] = cg.htr_in[t0 + k];
+    }
+}
+
 // The step as the handle API's own launches, domain by domain.
 template <class P>
-cudaError_t enqueue_domain(const DomainDev<P>& d, cudaStream_t st) {
-    const redi::StepForm form =
-        d.ts_first ? redi::step_form(d.rc.ntr, redi::cell_tuning(), false, d.cs.eos.variant) : redi::StepForm::kSeparate;
+cudaError_t enqueue_domain(const DomainDev<P>& d, const LaunchLayout& lay, cudaStream_t st) {
+    const int ntr = d.rc.ntr;
+    const redi::StepForm form = lay.ts_first ? redi::step_form(ntr, redi::cell_tuning(), false, d.cs.eos.variant)
+                                             : redi::StepForm::kSeparate;
     cudaError_t e;
-    if (!d.ts_first) {
+    if (form == redi::StepForm::kSeparate) {
         e = redi::launch_column_state(d.cs, st);
         if (e == cudaSuccess) e = redi::launch_sweep<P>(d.sw, st);
         if (e == cudaSuccess) e = redi::launch_phase_b<P>(d.rc, d.ff, d.cg, st, redi::Band{}, 0, 0, true);
         return e;
     }
-    const int swap = d.ts_first == 2 ? 1 : 0;
-    const bool flux = form != redi::StepForm::kSeparate;
-    e = redi::launch_column_recon<P>(d.cs, d.rc, swap, form, st);
-    if (e == cudaSuccess)
-        e = flux ? redi::launch_sweep_flux<P>(d.sw, d.ff, swap, form, st) : redi::launch_sweep<P>(d.sw, st);
-    if (e == cudaSuccess) e = redi::launch_phase_b<P>(d.rc, d.ff, d.cg, st, redi::Band{}, 2, flux ? 2 : 0, true);
-    return e;
+    const int swap = lay.ts_first == 2 ? 1 : 0;
+    redi::ReconArgsT<P> rc = d.rc;
+    redi::FaceFluxArgsT<P> ff = d.ff;
+    redi::CellGatherArgsT<P> cg = d.cg;
+    rc.ntr = 2;
+    ff.ppm = rc.ppm = reinterpret_cast<typename P::Ppm*>(lay.scratch + lay.ppm_ts);
+    flux_buffer(ff, cg, lay.scratch + lay.flux_ts, 2, 0, 2);
+    e = redi::launch_column_recon<P>(d.cs, rc, swap, form, st);
+    if (e == cudaSuccess) e = redi::launch_sweep_flux<P>(d.sw, ff, swap, form, st);
+    if (e == cudaSuccess) e = redi::launch_phase_b<P>(rc, ff, cg, st, redi::Band{}, 2, 2, true);
+    if (e != cudaSuccess || ntr == 2) return e;
+    rc = d.rc;
+    ff = d.ff;
+    cg = d.cg;
+    rc.ntr = ntr - 2;
+    for (int k = 0; k < rc.ntr; ++k) rc.htr[k] = d.rc.htr[2 + k];
+    rc.ti = reinterpret_cast<double*>(lay.scratch);
+    rc.ppm = reinterpret_cast<typename P::Ppm*>(lay.scratch + redi::recon_ppm_offset(rc.nx, rc.ny, rc.nz, rc.ntr));
+    ff.ti = rc.ti;
+    ff.ppm = rc.ppm;
+    flux_buffer(ff, cg, lay.scratch + up256(redi::recon_bytes<P>(rc.nx, rc.ny, rc.nz, rc.ntr)), lay.slots, 2, rc.ntr);
+    return redi::launch_phase_b<P>(rc, ff, cg, st, redi::Band{}, 0, 0, true);
 }
 
 template <class P>
@@ -617,7 +675,7 @@ cudaError_t enqueue_launches(redi_b200_batch* b, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaEventRecord(b->fork, st);
     for (size_t l = 0; l < b->lanes.size() && e == cudaSuccess; ++l) e = cudaStreamWaitEvent(b->lanes[l], b->fork, 0);
     for (int k : b->order)
-        if (e == cudaSuccess) e = enqueue_domain<P>(hd[k], b->lanes[b->lane_of[k]]);
+        if (e == cudaSuccess) e = enqueue_domain<P>(hd[k], b->layouts[k], b->lanes[b->lane_of[k]]);
     // joined even after an error: a capture must end with every stream back
     for (size_t l = 0; l < b->lanes.size(); ++l) {
         const cudaError_t r = cudaEventRecord(b->lane_done[l], b->lanes[l]);

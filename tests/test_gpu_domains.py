@@ -254,3 +254,72 @@ def test_batch_form_by_size(redi_lib, n, shape, npas, launches):
     for k, (x, y) in enumerate(zip(*out)):
         for i, (a, c) in enumerate(zip(x, y)):
             _assert_exact(f"domain {k} tracer {i}", a, c)
+
+
+@pytest.mark.parametrize("npas,eos,precision", [(0, 1, 0), (0, 2, 0), (1, 2, 1), (4, 1, 0), (6, 1, 1), (10, 2, 0)])
+def test_batch_memory(redi_lib, npas, eos, precision):
+    """A batch takes the bytes of the coefficients and of the phases one after the other (Phase A's state in
+    the bytes of Phase B's buffers, fluxes of two tracers), with T and S alone less than a tenth more."""
+    R = redi_lib
+    small = R.to_device(inputs.make_problem(12, 10, 4, n_passive=npas, seed=3))
+    b = R.RediBatch([small], precision=precision)  # the kernels are loaded
+    b.step()
+    b.destroy()
+    p = inputs.make_problem(260, 180, 40, n_passive=npas, seed=3)
+    dp = R.to_device(p)
+    dp.eos.variant = eos
+    nx, ny, nz, ntr = p.nx, p.ny, p.nz, p.ntr
+    faces, ncol, ns = (nx + 1) * ny + nx * (ny + 1), nx * ny, 2 * nz + 2
+    ko, f = (2, 4) if precision else (4, 8)
+    coef = faces * (ns * (16 + 2 * ko) + (ns - 1) * f + 1)
+    in_turn = max(40 * ncol * (nz + 1), ntr * ncol * (8 * (nz + 1) + 4 * f * nz) + 2 * (ns - 1) * faces * f)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    b = R.RediBatch([dp], precision=precision)
+    used = free - torch.cuda.mem_get_info()[0]
+    b.destroy()
+    assert used <= (coef + in_turn) * (1.1 if npas == 0 else 1.0) + (8 << 20), (used, coef + in_turn)
+
+
+@pytest.mark.parametrize("npas", [0, 1, 3, 7, 10])
+@pytest.mark.parametrize("setting", ["default", "group 1", "group 8", "sweep 3", "sweep 0", "gather 4", "gather 8",
+                                     "staged", "fold"])
+def test_batch_launches_under_other_settings(redi_lib, npas, setting):
+    """The launches per domain under every process-wide form, and with T and S in other places: the handle's
+    bits (its own tests compare those with the oracle)."""
+    from more_benchmarks_dc_ocean_b200 import autotune as T
+
+    R = redi_lib
+    ps = [inputs.make_problem(*s, n_seamounts=3, land_fraction=0.2, n_passive=npas, seed=70 + k)
+          for k, s in enumerate([(21, 17, 5), (19, 26, 27), (33, 8, 1)])]
+    ps[1].tracers[0], ps[1].tracers[1] = ps[1].tracers[1], ps[1].tracers[0]
+    ps[1].idx_temperature, ps[1].idx_salinity = 1, 0
+    if npas:
+        ps[2].tracers[1], ps[2].tracers[2] = ps[2].tracers[2], ps[2].tracers[1]
+        ps[2].idx_salinity = 2
+    want = [_handle_run(R, p, 2) for p in ps]
+    saved = (T.get_tracer_group(), T.get_sweep_form(), T.get_gather_tracers(), T.get_flux_staged(), T.get_fold(),
+             T.get_tuning())
+    try:
+        {"default": lambda: None, "group 1": lambda: T.set_tracer_group(1), "group 8": lambda: T.set_tracer_group(8),
+         "sweep 3": lambda: T.set_sweep_form(3), "sweep 0": lambda: T.set_sweep_form(0),
+         "gather 4": lambda: (T.set_tracer_group(4), T.set_gather_tracers(4, 1)),
+         "gather 8": lambda: (T.set_tracer_group(4), T.set_tuning(64, 2, 4), T.set_gather_tracers(8, 1)),
+         "staged": lambda: T.set_flux_staged(1), "fold": lambda: T.set_fold(T.FOLD_FP64)}[setting]()
+        dps = [R.to_device(p) for p in ps]
+        b = R.RediBatch(dps)
+        b.set_form(R.BATCH_LAUNCHES)
+        b.step(2)
+        st = b.status()
+        b.destroy()
+    finally:
+        T.set_tracer_group(saved[0])
+        T.set_sweep_form(saved[1])
+        T.set_tuning(*saved[5])
+        T.set_gather_tracers(*saved[2])
+        T.set_flux_staged(saved[3])
+        T.set_fold(*saved[4])
+    assert st["status"] == 0 and st["bad"] == 0, st
+    for p, dp, ref in zip(ps, dps, want):
+        for n, (t, c) in enumerate(zip(dp.ms.tracers, ref)):
+            _assert_exact(f"{setting} {p.name} tracer {n}", t.cpu().numpy(), c)
