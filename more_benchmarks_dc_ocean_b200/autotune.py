@@ -5,8 +5,9 @@ column in vertical chunks of `chunk` layers (see csrc/redi_plain.cu). Results
 are identical for every choice; speed is not: the tile sets how many
 neighbouring columns and face rows a block shares through L1, the chunk sets
 the L2 working set between the W, E, S and N passes against the lane
-divergence at chunk edges. The tuner times every candidate on the live problem
-with the library's own CUDA-event launch timing and keeps the fastest,
+divergence at chunk edges. The tuner times redi_apply_flux under every candidate
+on the live problem with the library's own CUDA-event timing (all of a call's
+kernels: the forms group tracers into launches differently) and keeps the fastest,
 caching it per (GPU name, domain size class, nz, tracer count, precision) in a
 JSON file (``$REDI_B200_TUNING_CACHE`` or ``~/.cache/redi_b200/tuning.json``).
 """
@@ -22,7 +23,6 @@ TILES: Tuple[Tuple[int, int], ...] = ((32, 4), (64, 2), (128, 1), (32, 2), (32, 
 CHUNKS: Tuple[int, ...] = (4, 8, 16)
 # Tiles of 128 threads also run the gather with its per-layer sums in shared memory.
 SMEM_TILES: Tuple[Tuple[int, int], ...] = ((32, 4), (64, 2), (128, 1))
-K_CELL_UPDATE = 3
 
 
 def _cache_path() -> str:
@@ -236,13 +236,13 @@ def _apply(cand) -> None:
 
 def tune(dp, redi, candidates: Optional[Iterable[Tuple[int, ...]]] = None, reps: int = 2,
          use_cache: bool = True, stream=None) -> dict:
-    """Time the cell update for every (bx, by, chunk[, smem]) candidate and keep the fastest.
+    """Time redi_apply_flux under every (bx, by, chunk[, smem]) candidate and keep the fastest.
 
     smem = 1 runs the gather with its per-layer sums in shared memory (128-thread tiles), 2 the same
     with 8 sublayers fetched per round trip, 3 with batches of 4 software-pipelined; 4 the row gather
     (one candidate: it has a shape of its own).
     Runs redi_apply_flux on ``dp`` (its tracers are advanced in place). Returns
-    {"best": (bx, by, chunk, smem), "ms": {candidate: ms per launch}, "cached": bool}.
+    {"best": (bx, by, chunk, smem), "ms": {candidate: ms of kernels per call}, "cached": bool}.
     """
     import torch
 
@@ -271,8 +271,7 @@ def tune(dp, redi, candidates: Optional[Iterable[Tuple[int, ...]]] = None, reps:
         kt = (C.c_double * R.lib().redi_b200_kernel_count())()
         kc = (C.c_ulonglong * R.lib().redi_b200_kernel_count())()
         R._check(L.redi_b200_profile_end(kt, kc, len(kt)))
-        kid = K_CELL_UPDATE
-        times[cand] = kt[kid] / max(1, kc[kid])
+        times[cand] = sum(kt) / reps  # by the call: the forms differ in how many launches share its work
     best = min(times, key=times.get)
     _apply(best)
     _store(dp, prec, best)
