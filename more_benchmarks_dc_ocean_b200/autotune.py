@@ -8,8 +8,8 @@ the L2 working set between the W, E, S and N passes against the lane
 divergence at chunk edges. The tuner times redi_apply_flux under every candidate
 on the live problem with the library's own CUDA-event timing (all of a call's
 kernels: the forms group tracers into launches differently) and keeps the fastest,
-caching it per (GPU name, domain size class, nz, tracer count, precision) in a
-JSON file (``$REDI_B200_TUNING_CACHE`` or ``~/.cache/redi_b200/tuning.json``).
+caching it per (GPU name, domain size class, nz, tracer count, precision, set of
+forms) in a JSON file (``$REDI_B200_TUNING_CACHE`` or ``~/.cache/redi_b200/tuning.json``).
 """
 
 from __future__ import annotations
@@ -192,13 +192,18 @@ def tune_tracer_group(dp, redi, reps: int = 2, stream=None) -> dict:
     return {"best": best, "ms": {f"flux{g}/gather{n}": round(v, 4) for (g, n), v in times.items()}}
 
 
+# The set of forms a cached choice was made from: raised with every form that tune() learns to time, so
+# that a choice made without it is not taken up again.
+FORMS = 2
+
+
 def _key(dp, precision: int) -> str:
     import torch
 
     name = torch.cuda.get_device_name(dp.ms.h_layer.device)
     cells = dp.grid.nx_total * dp.grid.ny_total
     size_class = "large" if cells >= 1 << 20 else ("medium" if cells >= 1 << 16 else "small")
-    return f"{name}|{size_class}|nz{dp.ms.nz_ml}|ntr{len(dp.ms.tracers)}|p{precision}"
+    return f"{name}|{size_class}|nz{dp.ms.nz_ml}|ntr{len(dp.ms.tracers)}|p{precision}|forms{FORMS}"
 
 
 def load_cached(dp, precision: int = 0) -> Optional[Tuple[int, int, int]]:

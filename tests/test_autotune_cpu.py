@@ -88,3 +88,17 @@ def test_forms_are_ranked_by_the_call(fake, ntr):
     res = autotune.tune(dp, types.SimpleNamespace(precision=0), candidates=[(64, 2, 8, 3), (64, 2, 8, 4)], use_cache=False)
     assert res["best"] == (64, 2, 8, 4) and lib.form == 4, res
     assert res["ms"]["64x2/ch8/rows"] == pytest.approx(0.8 * pairs + 1.0)
+
+
+def test_choices_of_an_older_set_of_forms_are_not_taken_up(fake, tmp_path):
+    """An entry stored before the row gather was known (three or four numbers) is timed anew, and the new
+    choice is found again."""
+    lib, dp = fake(2, lambda form, n: (1, 1.0 if form == 4 else 2.0))
+    for old in ([64, 2, 8], [64, 2, 8, 3]):
+        (tmp_path / "tuning.json").write_text(json.dumps({"fake|small|nz10|ntr2|p0": old}))
+        lib.form = 4
+        res = autotune.tune(dp, types.SimpleNamespace(precision=0), candidates=[(64, 2, 8, 3), (64, 2, 8, 4)])
+        assert not res["cached"] and res["best"] == (64, 2, 8, 4) and lib.form == 4, res
+        lib.form = 0
+        again = autotune.tune(dp, types.SimpleNamespace(precision=0))
+        assert again["cached"] and again["best"] == (64, 2, 8, 4) and lib.form == 4, again
