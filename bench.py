@@ -506,10 +506,17 @@ def _time_steps(dp, redi, st, warmup: int, steps: int) -> float:
     return e0.elapsed_time(e1) / steps
 
 
+# Gather shapes that win in either precision, the default form (last) among them.
+MIXED_SHAPES = [(64, 2, 4, 1), (64, 2, 8, 1), (32, 4, 8, 1), (32, 4, 16, 2), (64, 2, 16, 2), (64, 2, 16, 3), (32, 4, 8, 3),
+                (64, 2, 8, 4)]
+BATCHED_SHAPES = [(64, 2, 4, 0), (64, 2, 4, 1), (32, 4, 4, 1), (64, 2, 8, 1), (32, 4, 8, 1), (32, 4, 4, 2), (32, 4, 8, 2),
+                  (32, 4, 8, 3), (64, 2, 8, 3), (32, 4, 4, 3), (64, 2, 8, 4)]
+
+
 def _mixed_batched(args, p, dp, st, plain_value: float) -> dict:
     """Sub-records for the mixed+batched half of the metric, measured in this process right after the
     plain line: config 2 (the same 1440x1080x75 inputs, mixed precision) and config 3 (720x576x50, T, S
-    and 32 passive tracers, mixed precision, every tracer's fluxes in one fused Phase-B launch). Each
+    and 32 passive tracers, mixed precision). Each
     reports ms per step, tracer-cell updates/s and its ratio to the plain FP64 value of this line."""
     import torch
 
@@ -520,13 +527,11 @@ def _mixed_batched(args, p, dp, st, plain_value: float) -> dict:
 
     out = {}
     steps, warm = max(3, min(args.steps, 10)), 3
-    saved = (autotune.get_tuning(), autotune.get_gather_tracers())
+    saved = (autotune.get_tuning(), autotune.get_gather_tracers(), autotune.get_tracer_group())
     redi = R.make_redi(dp, R.MIXED)
-    # The FP64 line's gather shape is not the mixed one's best (FP32 fluxes halve the gather's
-    # loads), so the mixed step picks its own among the shapes that win in either precision.
-    shape2 = autotune.tune(dp, redi, candidates=[(64, 2, 4, 1), (64, 2, 8, 1), (32, 4, 8, 1), (32, 4, 16, 2),
-                                                   (64, 2, 16, 2), (64, 2, 16, 3), (32, 4, 8, 3)], reps=1,
-                           use_cache=False, stream=st)
+    # The FP64 line's gather shape need not be the mixed one's best (FP32 fluxes halve the gather's
+    # loads), so the mixed step picks its own.
+    shape2 = autotune.tune(dp, redi, candidates=MIXED_SHAPES, reps=1, use_cache=False, stream=st)
     ms = _time_steps(dp, redi, st, warm, steps)
     redi.destroy()
     upd = p.ntr * p.nx_phys * p.ny_phys * p.nz / (ms * 1e-3)
@@ -538,10 +543,7 @@ def _mixed_batched(args, p, dp, st, plain_value: float) -> dict:
     q = inputs.config3()
     dq = R.to_device(q, torch.device("cuda", torch.cuda.current_device()))
     redi = R.make_redi(dq, R.MIXED)
-    shape = autotune.tune(dq, redi, candidates=[(64, 2, 4, 0), (64, 2, 4, 1), (32, 4, 4, 1), (64, 2, 8, 1),
-                                                  (32, 4, 8, 1), (32, 4, 4, 2), (32, 4, 8, 2), (32, 4, 8, 3),
-                                                  (64, 2, 8, 3), (32, 4, 4, 3)], reps=1,
-                          use_cache=False, stream=st)
+    shape = autotune.tune(dq, redi, candidates=BATCHED_SHAPES, reps=1, use_cache=False, stream=st)
     group = autotune.tune_tracer_group(dq, redi, stream=st)
     ms = _time_steps(dq, redi, st, warm, steps)
     redi.destroy()
@@ -553,7 +555,7 @@ def _mixed_batched(args, p, dp, st, plain_value: float) -> dict:
                          "ms_per_step": ms, "value": upd, "unit": UNIT, "steps": steps, "warmup": warm,
                          "ratio_vs_plain": upd / plain_value, "tracer_group_ms": group["ms"],
                          "gather_shape": list(shape["best"]), "gather_shape_ms": shape["ms"]}
-    autotune.set_tracer_group(8)
+    autotune.set_tracer_group(saved[2])
     autotune.set_tuning(*saved[0])
     autotune.set_gather_tracers(saved[1][0], saved[1][1])
     del dq

@@ -1,0 +1,40 @@
+"""What bench.py reports beside its measured times, with the measured calls stubbed out."""
+
+import types
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import bench  # noqa: E402
+from more_benchmarks_dc_ocean_b200 import autotune as T, inputs  # noqa: E402
+
+
+def test_mixed_lines_try_the_default_gather_and_leave_the_forms_alone(redi_lib, monkeypatch):
+    """The mixed-precision lines choose among shapes that include the library's default gather, and the
+    process goes on with the forms it had."""
+    seen = []
+
+    def tune(dp, redi, candidates, **_):
+        seen.append(list(candidates))
+        T._apply(candidates[0])
+        return {"best": candidates[0], "ms": {}}
+
+    def tune_group(*_, **__):
+        T.set_tracer_group(8)
+        return {"best": (8, 2), "ms": {}}
+
+    p = inputs.make_problem(12, 10, 4, seed=1)
+    monkeypatch.setattr(T, "tune", tune)
+    monkeypatch.setattr(T, "tune_tracer_group", tune_group)
+    monkeypatch.setattr(bench, "_time_steps", lambda *a: 1.0)
+    monkeypatch.setattr(inputs, "config3", lambda: p)
+    monkeypatch.setattr(redi_lib, "make_redi", lambda *a: types.SimpleNamespace(destroy=lambda: None))
+    monkeypatch.setattr(redi_lib, "to_device", lambda *a: None)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "empty_cache", lambda: None)
+    before = (T.get_tuning(), T.get_gather_tracers(), T.get_tracer_group())
+    bench._mixed_batched(types.SimpleNamespace(steps=3), p, None, None, 1.0)
+    assert (T.get_tuning(), T.get_gather_tracers(), T.get_tracer_group()) == before
+    default = before[0] + (before[1][1],)
+    assert len(seen) == 2 and all(default in c for c in seen), seen
