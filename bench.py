@@ -57,7 +57,7 @@ UNIT = "tracer-cell updates/s"
 KERNEL_NAMES = ["k_column_state", "k_neutral_sweep", "k_tracer_recon", "k_cell_gather", "k_face_flux",
                 "k_mixed_recon", "k_mixed_flux", "k_mixed_sweep", "k_domain_persistent", "aux",
                 "k_meke_column", "k_meke_del2", "k_meke_lateral", "k_ale_columns", "k_ale_faces",
-                "k_flux_fold", "k_mixed_fold", "k_column_recon"]
+                "k_flux_fold", "k_mixed_fold", "k_column_recon", "k_sweep_flux", "k_mixed_sweep_flux", "k_batch_gate"]
 NKERN = len(KERNEL_NAMES)
 FALLBACK_HBM_GBS = 6650.0
 
@@ -690,7 +690,7 @@ def run_domains(args, rank, world, local_rank):
         stages = batch.stage_times()
         batch.set_accounting(False)
         ms_all = _max_over_ranks(ms, dist, dev)
-        k = 8  # k_domain_persistent
+        k = 20 if batch.get_form() == R.BATCH_LAUNCHES else 8  # k_batch_gate (the whole step) or k_domain_persistent
         bytes_launch = float(sum(boundary_bytes(p, name) for p in ps))
         t_launch = kt[k] / max(1, kc[k]) * 1e-3
         results[name] = {

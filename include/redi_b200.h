@@ -209,7 +209,11 @@ REDI_B200_API int redi_b200_version(void);
  * 8 domain_persistent, 9 auxiliary, and the MEKE step's (meke_b200.h) 10 pass A,
  * 11 biharmonic Laplacian, 12 pass B, and the ALE remap step's (ale_b200.h) 13 column
  * tiles, 14 face tiles, then 15 flux_fold and 16 mixed_fold (the fused Phase-B
- * pass); redi_b200_kernel_count() is their number.
+ * pass), 17 column_recon (column state and T/S reconstruction in one pass), 18
+ * sweep_flux and 19 mixed_sweep_flux (the sweep with the fluxes of T and S), 20
+ * the gate of a batch step made of launches per domain, whose launches count
+ * under their own ids and whose time is the whole step's;
+ * redi_b200_kernel_count() is their number.
  * redi_b200_launch_count(k) counts launches of kernel k since load (k < 0:
  * all). Between profile_begin and profile_end every launch is bracketed by a
  * CUDA event pair on its own stream; profile_end waits for them and returns,

@@ -287,7 +287,7 @@ def tune(dp, redi, candidates: Optional[Iterable[Tuple[int, ...]]] = None, reps:
 # Gather tiles of the persistent multi-domain kernel: its blocks are 128 threads.
 BATCH_TILES: Tuple[Tuple[int, int], ...] = ((32, 4), (16, 8))
 BATCH_OCCUPANCY: Tuple[int, ...] = (4, 5, 6)
-K_DOMAIN_PERSISTENT = 8
+K_DOMAIN_PERSISTENT, K_BATCH_LAUNCHES = 8, 20
 
 
 def tune_batch(batch, candidates: Optional[Iterable[Tuple[int, int, int]]] = None, reps: int = 2,
@@ -315,7 +315,7 @@ def tune_batch(batch, candidates: Optional[Iterable[Tuple[int, int, int]]] = Non
         kt = (C.c_double * R.lib().redi_b200_kernel_count())()
         kc = (C.c_ulonglong * R.lib().redi_b200_kernel_count())()
         R._check(L.redi_b200_profile_end(kt, kc, len(kt)))
-        return kt[K_DOMAIN_PERSISTENT] / max(1, kc[K_DOMAIN_PERSISTENT])
+        return (kt[K_DOMAIN_PERSISTENT] + kt[K_BATCH_LAUNCHES]) / reps
 
     times = {}
     batch.set_form(R.BATCH_PERSISTENT)

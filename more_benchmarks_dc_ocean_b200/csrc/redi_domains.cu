@@ -696,7 +696,7 @@ bool by_launches(const redi_b200_batch* b) {
 
 cudaError_t enqueue_any(redi_b200_batch* b, cudaStream_t st, bool instrument) {
     if (by_launches(b)) {
-        if (instrument) redi::launch_begin(redi::K_DOMAIN_PERSISTENT, st);
+        if (instrument) redi::launch_begin(redi::K_BATCH_LAUNCHES, st);
         cudaError_t e;
         {
             redi::LaunchTally tally;
@@ -705,7 +705,7 @@ cudaError_t enqueue_any(redi_b200_batch* b, cudaStream_t st, bool instrument) {
             std::copy(tally.n, tally.n + redi::K_NUM, b->tally);
         }
         if (instrument) {
-            redi::launch_end(redi::K_DOMAIN_PERSISTENT, st);
+            redi::launch_end(redi::K_BATCH_LAUNCHES, st);
             count_tally(b);
         }
         return e;
@@ -773,9 +773,10 @@ int redi_b200_batch_step(redi_b200_batch* b, void* stream) {
         if (e != cudaSuccess) return bfail(REDI_B200_E_CUDA, std::string("redi_b200_batch_step: graph: ") + cudaGetErrorString(e));
         b->exec_launches = launches;
     }
-    redi::launch_begin(redi::K_DOMAIN_PERSISTENT, st);
+    const int kid = launches ? redi::K_BATCH_LAUNCHES : redi::K_DOMAIN_PERSISTENT;
+    redi::launch_begin(kid, st);
     cudaError_t e = cudaGraphLaunch(b->exec, st);
-    redi::launch_end(redi::K_DOMAIN_PERSISTENT, st);
+    redi::launch_end(kid, st);
     count_tally(b);
     return e == cudaSuccess ? REDI_B200_OK : bfail(REDI_B200_E_CUDA, cudaGetErrorString(e));
 }

@@ -212,7 +212,10 @@ enum KernelId : int {
     K_FLUX_FOLD = 15,     // Phase B fused face flux + fold (FP64)
     K_MIXED_FOLD = 16,    // Phase B fused face flux + fold (mixed)
     K_COLUMN_RECON = 17,  // column state + T/S reconstruction in one pass (whole-step call)
-    K_NUM = 18
+    K_SWEEP_FLUX = 18,    // neutral sweep with the fluxes of T and S (whole-step call, FP64)
+    K_MIXED_SWEEP_FLUX = 19,
+    K_BATCH_LAUNCHES = 20,  // the gate of a batch step made of launches per domain; timed, the whole step
+    K_NUM = 21
 };
 
 // Sets the message redi_b200_last_error() returns on the calling thread.

@@ -403,7 +403,7 @@ cudaError_t launch_sweep_flux(const SweepArgsT<P>& sw, const FaceFluxArgsT<P>& f
     const BandRanges r = band_ranges(sw.nx, sw.ny, band);
     const unsigned nb = face_blocks(r.f);
     if (nb > 0) {
-        const int kid = P::kMixed ? K_MIXED_SWEEP : K_NEUTRAL_SWEEP;
+        const int kid = P::kMixed ? K_MIXED_SWEEP_FLUX : K_SWEEP_FLUX;
         launch_begin(kid, st);
         const cudaError_t e = form == StepForm::kFluxPacked
                                   ? launch_sweep_flux_t<P, true>(sw, ff, ts_swap, r.f, nb, st)

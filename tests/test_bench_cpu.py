@@ -38,3 +38,7 @@ def test_mixed_lines_try_the_default_gather_and_leave_the_forms_alone(redi_lib, 
     assert (T.get_tuning(), T.get_gather_tracers(), T.get_tracer_group()) == before
     default = before[0] + (before[1][1],)
     assert len(seen) == 2 and all(default in c for c in seen), seen
+
+
+def test_every_kernel_id_has_a_name(redi_lib):
+    assert len(bench.KERNEL_NAMES) == redi_lib.lib().redi_b200_kernel_count()

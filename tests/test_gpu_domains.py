@@ -323,3 +323,35 @@ def test_batch_launches_under_other_settings(redi_lib, npas, setting):
     for p, dp, ref in zip(ps, dps, want):
         for n, (t, c) in enumerate(zip(dp.ms.tracers, ref)):
             _assert_exact(f"{setting} {p.name} tracer {n}", t.cpu().numpy(), c)
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_batch_launch_counts(redi_lib, graph):
+    """The launch counter tells the sweep with fluxes from the plain one, and a step made of launches (its
+    gate, and every domain's under their own ids) from the persistent kernel."""
+    import ctypes as C
+
+    R = redi_lib
+    L = R.lib()
+    L.redi_b200_launch_count.restype = C.c_ulonglong
+    L.redi_b200_launch_count.argtypes = [C.c_int]
+
+    def counts(call):
+        before = [L.redi_b200_launch_count(k) for k in range(L.redi_b200_kernel_count())]
+        call()
+        return {k: n for k in range(len(before)) if (n := L.redi_b200_launch_count(k) - before[k])}
+
+    ps = [inputs.make_problem(21, 17, 5, seed=1), inputs.make_problem(16, 12, 7, seed=2)]
+    dps = [R.to_device(p) for p in ps]
+    b = R.RediBatch(dps, use_graph=graph)
+    b.set_form(R.BATCH_LAUNCHES)
+    b.step()
+    assert counts(b.step) == {20: 1, 17: 2, 18: 2, 3: 2}  # gate; columns, sweep with fluxes, gather of two domains
+    b.set_form(R.BATCH_PERSISTENT)
+    b.step()
+    assert counts(b.step) == {8: 1}
+    b.destroy()
+    redi = R.make_redi(dps[0])
+    assert counts(lambda: R.step(dps[0], redi, 1)) == {17: 1, 18: 1, 3: 1}
+    torch.cuda.synchronize()
+    redi.destroy()
