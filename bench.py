@@ -564,13 +564,20 @@ def _mixed_batched(args, p, dp, st, plain_value: float) -> dict:
 
 
 # ---------------------------------------------------------------------------
-# Uneven-domain batch (config4): one persistent kernel over a tile-work queue
+# Uneven-domain batch (config4): launches per domain, or one persistent kernel over a tile-work queue
 # ---------------------------------------------------------------------------
-def _domains_config_block(ps, args, world, prec_name):
+def _batch_form(launches: bool):
+    """(kernel id of the step's time, its name, the step in words) of a batch step made of launches per domain or of
+    the persistent kernel."""
+    return ((20, "every launch of the step (one graph)", "every domain's launches on a few streams") if launches else
+            (8, "k_domain_persistent", "one persistent kernel"))
+
+
+def _domains_config_block(ps, args, world, prec_name, launches):
     shapes = [(p.nx_phys, p.ny_phys, p.nz) for p in ps]
     return {
         "workload": f"config4: {len(ps)} uneven regional domains (nx, ny log-uniform in [64, 512], nz in "
-                    f"{{25, 50, 75}}), {ps[0].ntr} tracers each, {prec_name} Redi step, one persistent kernel "
+                    f"{{25, 50, 75}}), {ps[0].ntr} tracers each, {prec_name} Redi step, {_batch_form(launches)[2]}, "
                     "replayed from a CUDA graph" + (f", {world} ranks x {len(ps)} domains" if world > 1 else ""),
         "domains": len(ps), "tracers": ps[0].ntr, "cells": int(sum(a * b * c for a, b, c in shapes)),
         "nx_range": [min(a for a, _, _ in shapes), max(a for a, _, _ in shapes)],
@@ -673,11 +680,12 @@ def run_domains(args, rank, world, local_rank):
         if not args.no_tune:
             tuning = autotune.tune_batch(batch, reps=2, stream=st)
             if dist is not None:
-                t = torch.tensor(list(tuning["best"]), dtype=torch.int64, device=dev)
-                dist.broadcast(t, 0)
-                best = tuple(int(v) for v in t.tolist())
+                t = torch.tensor(list(tuning["best"]) + [tuning["form"]], dtype=torch.int64, device=dev)
+                dist.broadcast(t, 0)  # every rank uses rank 0's choice
+                *best, form = (int(v) for v in t.tolist())
                 batch.set_tuning(best[:2], best[2], best[3])
-                tuning["best"] = best
+                batch.set_form(form)
+                tuning["best"], tuning["form"] = tuple(best), form
         batch.step(args.warmup, st)
         torch.cuda.synchronize()
         clocks = ClockSampler(_uuid(local_rank)) if prec == prec_main else None
@@ -685,22 +693,25 @@ def run_domains(args, rank, world, local_rank):
             clocks.start()
         ms, kt, kc, launches = timed(batch, args.steps)
         clk = clocks.stop() if clocks else None
-        batch.set_accounting(True)  # one more (untimed) step with per-stage accounting
+        launches_form = batch.get_form() == R.BATCH_LAUNCHES  # of the timed steps
+        batch.set_accounting(True)  # one more (untimed) step with per-stage accounting, by the persistent kernel
         batch.step(1, st)
         stages = batch.stage_times()
         batch.set_accounting(False)
         ms_all = _max_over_ranks(ms, dist, dev)
-        k = 20 if batch.get_form() == R.BATCH_LAUNCHES else 8  # k_batch_gate (the whole step) or k_domain_persistent
+        k, kernel, _ = _batch_form(launches_form)
         bytes_launch = float(sum(boundary_bytes(p, name) for p in ps))
         t_launch = kt[k] / max(1, kc[k]) * 1e-3
         results[name] = {
             "value": batch.updates * world / (ms_all * 1e-3), "ms_per_step": ms_all, "kernel_ms": kt[k] / max(1, kc[k]),
-            "launches": launches, "bytes": bytes_launch, "achieved_gbs": bytes_launch / t_launch / 1e9,
+            "launches": launches, "launches_form": launches_form, "kernel": kernel,
+            "bytes": bytes_launch, "achieved_gbs": bytes_launch / t_launch / 1e9,
             "status": stat, "clocks": clk, "updates": batch.updates, "items": batch.items,
-            "stage_accounting_ms_summed_over_blocks": {k: {kk: round(vv, 3) if isinstance(vv, float) else vv
-                                                           for kk, vv in v.items()} for k, v in stages.items()},
-            "tuning": {"gather_tile": list(tuning["best"][:2]), "vertical_chunk": tuning["best"][2],
-                       "occupancy": tuning["best"][3],
+            "persistent_kernel_stage_accounting_ms_summed_over_blocks": {
+                k: {kk: round(vv, 3) if isinstance(vv, float) else vv for kk, vv in v.items()}
+                for k, v in stages.items()},
+            "tuning": {"form": _batch_form(launches_form)[2], "gather_tile": list(tuning["best"][:2]),
+                       "vertical_chunk": tuning["best"][2], "occupancy": tuning["best"][3],
                        "grid_blocks": batch.get_tuning()["grid"], "candidates_ms": tuning["ms"]} if tuning else
             batch.get_tuning(),
             "per_domain_max_rel_err_vs_fp64_1step": ({"max": max(err), "median": statistics.median(err),
@@ -750,8 +761,9 @@ def run_domains(args, rank, world, local_rank):
             "metric": METRIC, "value": main["value"], "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": main["ms_per_step"], "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64" if args.precision == "fp64" else "f64+f32", "data": "synthetic",
-            "config": _domains_config_block(ps, args, world, "plain FP64" if args.precision == "fp64" else "mixed"),
-            "roofline": {"bound": "hbm", "kernel": "k_domain_persistent", "achieved": main["achieved_gbs"],
+            "config": _domains_config_block(ps, args, world, "plain FP64" if args.precision == "fp64" else "mixed",
+                                            main["launches_form"]),
+            "roofline": {"bound": "hbm", "kernel": main["kernel"], "achieved": main["achieved_gbs"],
                          "peak": peak, "peak_source": peak_kind, "unit": "GB/s", "frac": main["achieved_gbs"] / peak,
                          "traffic": None, "algorithmic_bytes_per_launch": main["bytes"]},
             "side_by_side": {k: {kk: vv for kk, vv in v.items() if kk not in ("clocks", "e2e")}

@@ -42,3 +42,13 @@ def test_mixed_lines_try_the_default_gather_and_leave_the_forms_alone(redi_lib, 
 
 def test_every_kernel_id_has_a_name(redi_lib):
     assert len(bench.KERNEL_NAMES) == redi_lib.lib().redi_b200_kernel_count()
+
+
+@pytest.mark.parametrize("launches", [False, True])
+def test_the_batch_line_names_the_form_it_timed(launches):
+    ps = [inputs.make_problem(12, 10, 4, seed=1)]
+    kid, kernel, words = bench._batch_form(launches)
+    block = bench._domains_config_block(ps, types.SimpleNamespace(precision="fp64"), 1, "plain FP64", launches)
+    assert words in block["workload"] and ("persistent" in block["workload"]) == (not launches)
+    assert bench.KERNEL_NAMES[kid] == ("k_batch_gate" if launches else "k_domain_persistent")
+    assert ("persistent" in kernel) == (not launches)
