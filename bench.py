@@ -102,8 +102,9 @@ def boundary_bytes(p, precision: str = "fp64") -> float:
     return 8 * s["Nt"] * (3 + 1 + 2 * s["ntr"]) + 2 * bcoef + b2d
 
 
-def kernel_bytes(p, kid: int, precision: str = "fp64") -> float:
-    """Algorithmic bytes one launch of kernel `kid` must move (its share of the boundary model)."""
+def kernel_bytes(p, kid: int, precision: str = "fp64", per_step: float = 1.0) -> float:
+    """Algorithmic bytes one launch of kernel `kid` must move (its share of the boundary model), with
+    `per_step` launches of it in a step."""
     s = _sizes(p)
     per_surf = 32 if precision == "fp64" else 24
     bcoef = (s["Fu"] + s["Fv"]) * s["ns"] * per_surf
@@ -116,12 +117,14 @@ def kernel_bytes(p, kid: int, precision: str = "fp64") -> float:
         return 8.0 * s["Nt"] * (1 + s["ntr"])
     if kid in (4, 6):  # face flux: read the coefficients once for every tracer
         return float(bcoef + face2d)
-    if kid == 3:       # cell gather, one launch per tracer pair: read + write its tracers
-        return float(16 * s["Nt"] * min(2, s["ntr"]) + 8 * s["ncol"])
+    if kid == 3:       # cell gather: read + write its share of the tracers
+        return float(16 * s["Nt"] * s["ntr"] / per_step + 8 * s["ncol"])
     if kid in (15, 16):  # fused face flux + fold: the coefficients once, every tracer read + written
         return float(bcoef + face2d + 16 * s["Nt"] * s["ntr"])
     if kid == 17:        # column state + T/S reconstruction in one pass: read h, T, S once
         return 24.0 * s["Nt"]
+    if kid in (18, 19):  # sweep with the fluxes of T and S: write the coefficients, which it does not read back
+        return float(bcoef + face2d)
     return 0.0
 
 
@@ -427,7 +430,7 @@ def run_b200(args, rank, world, local_rank):
                               "ms_per_launch": ktime[k] / kcount[k]} for k in range(NKERN) if kcount[k]}
     top = max((k for k in range(NKERN) if kcount[k]), key=lambda k: ktime[k])
     peak, peak_kind = _peaks()
-    bytes_launch = kernel_bytes(p, top, args.precision)
+    bytes_launch = kernel_bytes(p, top, args.precision, kcount[top] / args.steps)
     t_launch = ktime[top] / kcount[top] * 1e-3
     achieved = bytes_launch / t_launch / 1e9
     traffic = _ncu_traffic().get(KERNEL_NAMES[top]) if (p.nx_phys, p.ny_phys, p.nz) == (1440, 1080, 75) else None

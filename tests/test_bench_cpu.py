@@ -52,3 +52,21 @@ def test_the_batch_line_names_the_form_it_timed(launches):
     assert words in block["workload"] and ("persistent" in block["workload"]) == (not launches)
     assert bench.KERNEL_NAMES[kid] == ("k_batch_gate" if launches else "k_domain_persistent")
     assert ("persistent" in kernel) == (not launches)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_kernel_bytes_of_a_step(precision):
+    """The kernels of a whole step: the coefficients are written once, by the sweep with fluxes; the gather's
+    launches, however many, read and write every tracer once."""
+    p = inputs.make_problem(30, 20, 6, n_passive=7, seed=2)
+    by = lambda name, n=1.0: bench.kernel_bytes(p, bench.KERNEL_NAMES.index(name), precision, n)  # noqa: E731
+    surf = ((p.nx + 1) * p.ny + p.nx * (p.ny + 1)) * (2 * p.nz + 2) * (32 if precision == "fp64" else 24)
+    sweep = by("k_sweep_flux" if precision == "fp64" else "k_mixed_sweep_flux")
+    assert surf < sweep < 1.2 * surf
+    cells = p.nx * p.ny
+    for launches in (1, 2, 5):
+        assert launches * by("k_cell_gather", launches) == pytest.approx(16 * cells * p.nz * p.ntr + 8 * cells * launches)
+
+
+def test_measured_traffic_is_of_kernels_that_a_step_launches():
+    assert set(bench._ncu_traffic()) == {"k_column_recon", "k_sweep_flux", "k_cell_gather"}
