@@ -35,10 +35,10 @@
 // instead, on one thread, from the same tile. The column total is the last old
 // interface depth: the same additions in the same order.
 // What bounds both kernels is instruction issue and the latency of FP64 chains at
-// 16-24 warps per SM (shared memory holds whole columns), not bytes: 860 and 1010
-// thread instructions per (column, layer) of two fields, a third of them FP64,
-// against 2250 with one thread per (column, new layer) that searched, divided and
-// evaluated the parabola anew for every piece and field. k_ale_columns (T, S) and
+// 23 and 30 warps per SM (shared memory holds whole columns), not bytes: 790 and
+// 900 thread instructions per (column, layer) of two fields, issued in 47 and 67 %
+// of the cycles, against about 2000 with one thread per (column, new layer) that
+// searched, divided and evaluated the parabola anew for every piece and field. k_ale_columns (T, S) and
 // k_ale_faces at 479x303x30: 404 -> 222 us and 355 -> 181 us; at 1444x1084x75:
 // 19.2 -> 6.8 ms and 16.6 -> 6.1 ms (0.30 and 0.14 of the bytes' time at 6537 GB/s).
 // Compiled with -fmad=false: results are the reference's IEEE sequence.

@@ -2258,14 +2258,15 @@ __device__ __forceinline__ void st_sums(char* p, const LaneSums<NT>& r) {
     else *reinterpret_cast<double*>(p) = r.v[0];
 }
 
-// One face's sublayers of the chunk [k0, k0 + ch) from sublayer s on (the same
-// for the whole warp); `on`: this lane has the face. first: the lane's first
-// sublayer not yet added. Returns the next chunk's s. Every lane must call it.
-// The left face's column gains its fluxes, the right one's loses them: `sign`
-// is the sign bit to flip, an addition of -f being the subtraction of f.
+// f, or -f where `sign` is the sign bit.
 __device__ __forceinline__ double flip(double f, int sign) {
     return __hiloint2double(__double2hiint(f) ^ sign, __double2loint(f));
 }
+// One face's sublayers of the chunk [k0, k0 + ch) from sublayer s on (the same
+// for the whole warp); `on`: this lane has the face. first: the lane's first
+// sublayer not yet added. Returns the next chunk's s. Every lane must call it.
+// The column left of a face gains its fluxes, the one right of it loses them:
+// `sign` is the sign bit to flip, an addition of -f being the subtraction of f.
 template <int NT, class P, class LD, int U>
 __device__ __forceinline__ int gather_walk_rows(const typename P::Flux* __restrict__ F, unsigned f_stride,
                                                 const typename P::Ko* __restrict__ KoS, unsigned fo, unsigned stride,

@@ -336,17 +336,17 @@ cudaError_t launch_column_recon(const ColumnStateArgs& cs, const ReconArgsT<P>& 
 // S and T when ts_swap) into flux slots 0 and 1.
 template <class P>
 cudaError_t launch_sweep_flux(const SweepArgsT<P>& sw, const FaceFluxArgsT<P>& ff, int ts_swap, StepForm form,
-                              cudaStream_t st, Band band = Band{});
+                              cudaStream_t st);
 // Density and dSV/dT, dSV/dS at n points (T, S, p device arrays).
 cudaError_t launch_eos_points(const EosParams& e, int n, const double* T, const double* S, const double* p,
                               double* rho, double* dsv_dt, double* dsv_ds, cudaStream_t st);
 template <class P>
 cudaError_t launch_sweep(const SweepArgsT<P>& sw, cudaStream_t st, Band band = Band{});
-template <class P>
 // recon_from: the first tracer of rc to reconstruct (tracers before it were
 // reconstructed already, by launch_column_recon). flux_from: 2 when the fluxes
 // of tracers 0 and 1 are in flux slots 0 and 1 already (launch_sweep_flux).
 // no_fold: the fused fold is left out. ff.slots bounds the tracers per launch.
+template <class P>
 cudaError_t launch_phase_b(const ReconArgsT<P>& rc, const FaceFluxArgsT<P>& ff, const CellGatherArgsT<P>& cg,
                            cudaStream_t st, Band band = Band{}, int recon_from = 0, int flux_from = 0,
                            bool no_fold = false);

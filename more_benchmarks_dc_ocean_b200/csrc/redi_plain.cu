@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kSweepWinThreads) k_neutral_sweep_w(SweepArgsT
 
 // The same sweep with the fluxes of T and S evaluated as its surfaces are
 // placed (FluxSink). Bound by the instructions and dependent chains of a step
-// (480 warp instructions, half of its cycles issue one), then by what it reads
+// (430 warp instructions a surface, issued in 54 % of the cycles), then by what it reads
 // through L2. 1440x1080x75 FP64: 7.8 ms for the sweep and both fluxes, against
 // 5.3 + 7.2 ms in launches of their own. On the way there: layers requested at
 // the end of the step before 9.7 ms, unconditionally 9.8, not at all 7.0; the
@@ -399,8 +399,8 @@ static cudaError_t launch_sweep_flux_t(const SweepArgsT<P>& sw, const FaceFluxAr
 
 template <class P>
 cudaError_t launch_sweep_flux(const SweepArgsT<P>& sw, const FaceFluxArgsT<P>& ff, int ts_swap, StepForm form,
-                              cudaStream_t st, Band band) {
-    const BandRanges r = band_ranges(sw.nx, sw.ny, band);
+                              cudaStream_t st) {
+    const BandRanges r = band_ranges(sw.nx, sw.ny, Band{});
     const unsigned nb = face_blocks(r.f);
     if (nb > 0) {
         const int kid = P::kMixed ? K_MIXED_SWEEP_FLUX : K_SWEEP_FLUX;
@@ -414,9 +414,9 @@ cudaError_t launch_sweep_flux(const SweepArgsT<P>& sw, const FaceFluxArgsT<P>& f
     return cudaGetLastError();
 }
 template cudaError_t launch_sweep_flux<PlainPrec>(const SweepArgsT<PlainPrec>&, const FaceFluxArgsT<PlainPrec>&, int,
-                                                  StepForm, cudaStream_t, Band);
+                                                  StepForm, cudaStream_t);
 template cudaError_t launch_sweep_flux<MixedPrec>(const SweepArgsT<MixedPrec>&, const FaceFluxArgsT<MixedPrec>&, int,
-                                                  StepForm, cudaStream_t, Band);
+                                                  StepForm, cudaStream_t);
 
 template <int GNT, class P>
 static void launch_gather(const CellGatherArgsT<P>& cg, int tr, int slot, const BandRanges& r, const CellTuning& tune,
@@ -524,9 +524,6 @@ static void launch_flux(const FaceFluxArgsT<P>& ff, int tr0, const BandRanges& r
     launch_end(kid, st);
 }
 
-// The gathers of tracers tr0 .. tr0+NS-1, whose fluxes sit in slots 0 .. NS-1:
-// one launch of 8 tracers (WIDE: the fluxes of two face-flux launches), or
-// launches of 4 or 2 tracers, which read consecutive slots.
 // The row gathers of n tracers from tr0 on, whose fluxes sit in slots 0 .. n-1:
 // pairs, and an odd last tracer alone.
 template <class P>
@@ -536,6 +533,9 @@ static void launch_row_gathers(const CellGatherArgsT<P>& cg, int tr0, int n, con
     if (n & 1) launch_gather_rows<1, P>(cg, tr0 + n - 1, n - 1, r, st);
 }
 
+// The gathers of tracers tr0 .. tr0+NS-1, whose fluxes sit in slots 0 .. NS-1:
+// the row gathers, one launch of 8 tracers (WIDE: the fluxes of two face-flux
+// launches), or launches of 4 or 2 tracers, which read consecutive slots.
 template <int NS, class P, bool WIDE = false>
 static void launch_gathers(const CellGatherArgsT<P>& cg, int tr0, const BandRanges& r, const CellTuning& tune,
                            cudaStream_t st) {
