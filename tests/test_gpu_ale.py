@@ -188,3 +188,12 @@ def test_launches_counted(A, redi_lib):
     torch.cuda.synchronize()
     after = [L.redi_b200_launch_count(k) for k in (13, 14)]
     assert [b - a for a, b in zip(before, after)] == [4, 2]
+
+
+@pytest.mark.parametrize("nz", [35, 36, 42, 47, 48, 65, 72, 73, 83, 84, 96, 97])
+@pytest.mark.parametrize("method", [AI.REMAP_PCM, AI.REMAP_PLM, AI.REMAP_PPM])
+@pytest.mark.parametrize("n_passive", [-1, 0])
+def test_tile_edges_of_every_array_count(A, nz, method, n_passive):
+    """The depths on either side of each change of the tile width for tiles of 6, 7, 8 and 9 arrays: a tile is
+    32 columns wide up to nz 47, 41, 35 and 31 and 16 up to 96, 83, 72 and 64."""
+    test_tile_edges_and_serial_columns(A, nz, method, n_passive)

@@ -355,3 +355,48 @@ def test_batch_launch_counts(redi_lib, graph):
     assert counts(lambda: R.step(dps[0], redi, 1)) == {17: 1, 18: 1, 3: 1}
     torch.cuda.synchronize()
     redi.destroy()
+
+
+@pytest.mark.parametrize("form", ["persistent", "launches"])
+def test_batch_forms_match_oracle(redi_lib, oracle_lib, form):
+    """Two steps of uneven domains with every equation of state, in either form: the oracle's bits."""
+    R = redi_lib
+    ps = _domains()
+    for k, p in enumerate(ps):
+        p.eos.variant = (1, 2, 4)[k % 3]
+    dps = [R.to_device(p) for p in ps]
+    b = R.RediBatch(dps)
+    b.set_form(R.BATCH_PERSISTENT if form == "persistent" else R.BATCH_LAUNCHES)
+    b.step(2)
+    st = b.status()
+    b.destroy()
+    assert st["status"] == 0 and st["bad"] == 0, st
+    for p, dp in zip(ps, dps):
+        q = p.copy()
+        O.step(q, 2)
+        for n, (t, c) in enumerate(zip(dp.ms.tracers, q.tracers)):
+            _assert_exact(f"{p.name} eos {p.eos.variant} tracer {n}", t.cpu().numpy(), c)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_persistent_kernel_times_out_and_recovers(redi_lib, precision):
+    """The persistent kernel's bounded waits: the held domain is named, its tracers stay, and the next step
+    runs from where the others are."""
+    R = redi_lib
+    ps = _domains()[:4]
+    dps = [R.to_device(p) for p in ps]
+    b = R.RediBatch(dps, precision=precision)
+    b.set_form(R.BATCH_PERSISTENT)
+    b.set_wait_limit(100_000_000)  # 100 ms: the other domains take a fraction of one
+    b.hold(3)
+    b.step()
+    st = b.status()
+    assert st["status"] == R.STATUS_TIMEOUT and st["domain"] == 3 and st["stage"] in (0, 1), st
+    b.hold(3, False)
+    b.step()
+    assert b.status()["status"] == 0
+    b.destroy()
+    for k, (p, dp) in enumerate(zip(ps, dps)):
+        ref = _handle_run(R, p, 1 if k == 3 else 2, precision)
+        for n, (t, c) in enumerate(zip(dp.ms.tracers, ref)):
+            _assert_exact(f"{p.name} tracer {n}", t.cpu().numpy(), c)

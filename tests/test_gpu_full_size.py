@@ -131,3 +131,24 @@ def test_config4_largest_domains_match_oracle(redi_lib, oracle_lib):
         O.step(q, 1)
         for n in range(p.ntr):
             _exact(f"config4 {p.name} tracer {n}", dp.ms.tracers[n].cpu().numpy(), q.tracers[n])
+
+
+def test_largest_domains_in_the_persistent_kernel(redi_lib):
+    """The same domains in the batch's other form: the launches' bits (which the oracle's test compares)."""
+    R = redi_lib
+    shapes = inputs.config4_shapes()
+    order = sorted(range(len(shapes)), key=lambda d: -shapes[d][0] * shapes[d][1] * shapes[d][2])[:3]
+    ps = [inputs.config4_domain(20261203, d, shapes[d]) for d in order]
+    out = []
+    for form in (R.BATCH_LAUNCHES, R.BATCH_PERSISTENT):
+        dps = [R.to_device(p) for p in ps]
+        b = R.RediBatch(dps)
+        b.set_form(form)
+        b.step(1)
+        st = b.status()
+        b.destroy()
+        assert st["status"] == 0 and st["bad"] == 0, st
+        out.append([[t.cpu().numpy() for t in dp.ms.tracers] for dp in dps])
+    for p, x, y in zip(ps, *out):
+        for n in range(p.ntr):
+            _exact(f"{p.name} tracer {n}", y[n], x[n])
