@@ -361,10 +361,19 @@ cudaError_t launch_sweep(const SweepArgsT<P>& sw, cudaStream_t st, Band band) {
 // 4.85. 720x576x50 mixed, 34 tracers: batches of 6, chunks of 17 9.46 ms, 25
 // 10.62; batches of 8, 17 11.57; the thread-paced walk's best 11.47. A nz up
 // to the bound is one chunk (128x96x25: 0.040 ms; 13 layers 0.047), a larger one is cut evenly.
+// Up to kFew layers a face has fewer sublayers than two batches, most of what the
+// batches read ahead is not there, and the thread-paced walk is the faster one: 1000x800
+// FP64, T and S, rows and threads: nz 1 0.136 and 0.058 ms, 3 0.146 and 0.105, 5 0.203
+// and 0.154, 6 0.208 and 0.187 (300x200: 0.031 and 0.033); mixed 1 0.097 and 0.056, 3
+// 0.135 and 0.107, 4 0.140 and 0.136 (300x200: 0.019 and 0.023). Not where the cells
+// leave SMs without a warp: there it is the round trips and launches that count (5x4x3,
+// 4 tracers, both calls: 0.054 and 0.060 ms).
 template <class P>
 struct RowGather {
     static constexpr int kBatch = P::kMixed ? 6 : 8;
     static constexpr int kChunk = P::kMixed ? 19 : 25;
+    static constexpr int kFew = P::kMixed ? 3 : 5;
+    static constexpr int kFewCells = 148 * plain::kGatherRowThreads;
 };
 
 template <int NT, class P>
@@ -525,10 +534,20 @@ static void launch_flux(const FaceFluxArgsT<P>& ff, int tr0, const BandRanges& r
 }
 
 // The row gathers of n tracers from tr0 on, whose fluxes sit in slots 0 .. n-1:
-// pairs, and an odd last tracer alone.
+// pairs, and an odd last tracer alone; over a few layers the thread-paced walk
+// (RowGather::kFew) of the same.
 template <class P>
 static void launch_row_gathers(const CellGatherArgsT<P>& cg, int tr0, int n, const BandRanges& r, cudaStream_t st) {
     if (r.j1 <= r.j0) return;
+    if (cg.nz <= RowGather<P>::kFew && (r.j1 - r.j0) * cg.nx >= RowGather<P>::kFewCells) {
+        CellTuning walk;
+        walk.bx = 64, walk.by = 2, walk.chunk = 8, walk.gather_smem = 1;
+        const dim3 block(walk.bx, walk.by);
+        const dim3 grid((cg.nx + walk.bx - 1) / walk.bx, (r.j1 - r.j0 + walk.by - 1) / walk.by);
+        for (int g = 0; g + 1 < n; g += 2) launch_gather<2, P>(cg, tr0 + g, g, r, walk, grid, block, st);
+        if (n & 1) launch_gather<1, P>(cg, tr0 + n - 1, n - 1, r, walk, grid, block, st);
+        return;
+    }
     if (n > 1) launch_gather_rows<2, P>(cg, tr0, 0, r, st, n / 2);
     if (n & 1) launch_gather_rows<1, P>(cg, tr0 + n - 1, n - 1, r, st);
 }

@@ -598,3 +598,30 @@ def test_whole_step_call_gates(redi_lib):
     assert R.redi_step(dp.grid, dp.metrics, dp.eos, redi, dp.ms, dp.dt, dp.khtr_u_ext, dp.khtr_v_ext,
                        dp.bc) == R.SKIPPED
     redi.destroy()
+
+
+@pytest.mark.parametrize("nz", [1, 2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("npas,precision", [(0, 0), (1, 0), (3, 0), (0, 1), (1, 1), (6, 1)])
+def test_gather_of_a_few_layers(redi_lib, oracle_lib, nz, npas, precision):
+    """Either side of the depth below which the default gather walks thread by thread: the oracle's bits, and
+    in mixed precision those of the walk with its sums in registers; also with a slot for one tracer only."""
+    from more_benchmarks_dc_ocean_b200 import autotune
+
+    R = redi_lib
+    p = inputs.make_problem(167, 31, nz, n_passive=npas, seed=40 + nz)  # 171 x 35 cells: a warp for every SM
+
+    def run(group, form):
+        autotune.set_tracer_group(group)
+        autotune.set_gather_tracers(2, form)
+        dp = R.to_device(p)
+        redi = R.make_redi(dp, precision)
+        R.step(dp, redi, 2)
+        torch.cuda.synchronize()
+        assert redi.error_count() == 0
+        redi.destroy()
+        return [t.cpu().numpy() for t in dp.ms.tracers]
+
+    want = _run_oracle(p, 2)[1] if precision == 0 else run(2, 0)
+    for group in (2, 1):
+        for n, (a, b) in enumerate(zip(run(group, 4), want)):
+            _assert_exact(f"nz {nz} group {group} tracer {n}", a, b)
