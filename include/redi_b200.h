@@ -243,14 +243,14 @@ REDI_B200_API int redi_b200_get_tracer_group(void);
 
 /* Tracers one cell-gather launch folds (2, 4 or 8; default 2) and where it
  * walks (smem = 4, the default: a warp on whole rows of sublayers, in pairs of
- * tracers and chunks of its own, sums in shared memory; the others let each
- * thread walk at its own pace and differ in where a chunk's per-layer sums
- * live: 1: the thread's slots in shared memory, one load-add-store per flux; 2: the same, fetching 8
- * sublayers per round trip instead of 3 or 4; 3: the same with batches of 4
- * software-pipelined, the next batch in flight while one is folded; 0:
- * registers, a select-add over the chunk), process-wide (no counterpart in the
- * reference). 4 tracers read
- * the cell-side Ko half as often as 2. 8 folds the fluxes of two face-flux
+ * tracers and chunks of its own, sums in shared memory, and over a few layers as
+ * form 1; the others let each thread walk at its own pace and differ in where a
+ * chunk's per-layer sums live: 1: the thread's slots in shared memory, one
+ * load-add-store per flux; 2: the same, fetching 8 sublayers per round trip
+ * instead of 3 or 4; 3: the same with batches of 4 software-pipelined, the next
+ * batch in flight while one is folded; 0: registers, a select-add over the
+ * chunk), process-wide (no counterpart in the reference). 4 tracers read the
+ * cell-side Ko half as often as 2. 8 folds the fluxes of two face-flux
  * launches of 4 tracers in one walk; it applies with face-flux groups of 4,
  * shared-memory sums, 4-layer chunks and 128-thread tiles (else 4 is used).
  * Results do not depend on either choice.
@@ -369,16 +369,17 @@ REDI_B200_API int redi_b200_halo_copy(double* const* fields, int nfields, int nx
                                       double* buf, int to_buf, void* stream);
 
 /* ---------------------------------------------------------------------------
- * Many independent regional domains stepped together (no
- * counterpart in the reference, whose driver steps one domain per call). The
- * step of every domain (redi_calc_coeffs then redi_apply_flux for all of its
- * tracers) is cut into tiles of columns, faces and cells; one grid of resident
- * blocks drains that work queue, largest domains first, each tile starting
- * once the previous stage of its own domain is complete. Per domain the
- * results equal those of redi_b200_calc_coeffs + redi_b200_apply_flux on a
- * handle of the same precision, bit for bit.
+ * Many independent regional domains stepped together (no counterpart in the
+ * reference, whose driver steps one domain per call). A step takes one of two
+ * forms (redi_b200_batch_set_form): the handle API's launches for every domain
+ * on a few streams; or one persistent kernel, for which the step of every
+ * domain is cut into tiles of columns, faces and cells, and one grid of
+ * resident blocks drains that work queue, largest domains first, each tile
+ * starting once the previous stage of its own domain is complete. Per domain
+ * the results equal those of redi_b200_calc_coeffs + redi_b200_apply_flux on a
+ * handle of the same precision, bit for bit, in either form.
  * ------------------------------------------------------------------------- */
-#define REDI_B200_STATUS_TIMEOUT 1 /* a tile waited longer than the wait limit */
+#define REDI_B200_STATUS_TIMEOUT 1 /* something waited longer than the wait limit */
 
 /* One domain: what redi_b200_calc_coeffs and redi_b200_apply_flux take. The
  * per-face diffusivities are required (khtr_u_ext / khtr_v_ext non-NULL); ms
@@ -399,10 +400,12 @@ typedef struct redi_b200_batch redi_b200_batch;
 
 /* Builds the batch: Phase-A coefficient slots and scratch per domain, the work
  * queue, and the persistent grid (as many 128-thread blocks as are resident on
- * the current device). tile_bx x tile_by (= 128) is the cell tile of the
- * gather, chunk (4, 8, 16) its vertical chunk. use_graph != 0 captures the step
- * (counter reset + persistent kernel) in a CUDA graph on the first
- * redi_b200_batch_step and replays it afterwards. Synchronises the device. */
+ * the current device). tile_bx x tile_by (= 128) is the persistent kernel's cell
+ * tile of the gather, chunk (4, 8, 16) its vertical chunk. use_graph != 0
+ * captures the step in a CUDA graph on the first redi_b200_batch_step, and anew
+ * when its form changes, and replays it otherwise; a graph of launches keeps the
+ * process-wide kernel forms (redi_b200_set_sweep_form and the like) that were in
+ * force at its capture. Synchronises the device. */
 REDI_B200_API int redi_b200_batch_create(int ndomains, const redi_b200_domain* domains, int precision, int tile_bx,
                                          int tile_by, int chunk, int use_graph, redi_b200_batch** out);
 
@@ -414,7 +417,9 @@ REDI_B200_API int redi_b200_batch_step(redi_b200_batch* b, void* stream);
  * 1 neutral sweep, 2 tracer reconstruction, 3 + 2g / 4 + 2g face flux / gather
  * of tracer pair g) of the first tile that gave up; bad = fluxes the gather
  * found out of order (0 for coefficients made in the step). Any out pointer
- * but status may be NULL. After a timeout the step's results are incomplete. */
+ * but status may be NULL. After a timeout the step's results are incomplete. The
+ * launches wait at one place, a gate before the first of them: a step that times
+ * out there reports stage 0 and has changed nothing. */
 REDI_B200_API int redi_b200_batch_status(const redi_b200_batch* b, int* status, int* domain, int* stage, int* bad);
 
 /* Launch shape of an existing batch (tile and chunk as in
@@ -449,12 +454,14 @@ REDI_B200_API int redi_b200_batch_set_accounting(redi_b200_batch* b, int on);
 REDI_B200_API int redi_b200_batch_stage_times(const redi_b200_batch* b, double* wait_ms, double* busy_ms,
                                               long long* tiles);
 
-/* Longest time a tile waits for its predecessors, in ns (default 2e9). */
+/* Longest time a tile waits for its predecessors, or the gate of a step made of
+ * launches for a held domain, in ns (default 2e9). */
 REDI_B200_API int redi_b200_batch_set_wait_limit(redi_b200_batch* b, long long ns);
 
 /* Fault injection for tests: hold != 0 keeps the domain's first stage waiting
  * on a release flag that nothing sets while the step runs, so the step ends
- * with REDI_B200_STATUS_TIMEOUT after the wait limit. */
+ * with REDI_B200_STATUS_TIMEOUT after the wait limit. In the form AUTO the other
+ * domains go on meanwhile; with LAUNCHES the step stops before any of them. */
 REDI_B200_API int redi_b200_batch_hold(redi_b200_batch* b, int domain, int hold);
 
 /* Tracer-cell updates per step (physical cells x layers x tracers, summed),

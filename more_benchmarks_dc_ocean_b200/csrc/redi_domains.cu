@@ -11,8 +11,8 @@
 // accounting; on request): a step of every domain (Phase A then Phase B, all
 // tracers) is cut into work items: tiles of columns (interface state, tracer
 // reconstruction), tiles of faces (neutral sweep, face fluxes of one tracer
-// pair) and 2-D tiles of cells (the ordered gather of one tracer pair). The host builds the item queue once:
-// stage by stage, and within a stage domain by domain, largest domain first
+// pair) and 2-D tiles of cells (the ordered gather of one tracer pair). The host
+// builds the item queue once: stage by stage, and within a stage domain by domain, largest domain first
 // (longest-processing-time order), so an item's predecessors always sit earlier
 // in the queue. One persistent grid (as many blocks as fit on the GPU at once)
 // claims items through an atomic cursor.
@@ -396,7 +396,8 @@ int layout_any(redi_b200_batch* b) {
 }
 
 // Streams of the launches per domain: 12 domains of 64x64x25 take 0.51 / 0.41 / 0.31 / 0.26 ms on 3 / 5 / 8 /
-// 12 of them, 12 of up to 512x512x75 14.9 / 14.6 / 14.7 / 14.4.
+// 12 of them, 12 of up to 512x512x75 14.9 / 14.6 / 14.7 / 14.4 (FP64; the latter in mixed precision 16.9 on 12,
+// 15.1 on one).
 constexpr int kLanes = 12;
 
 // Launches of one domain's step: columns, sweep, gather; with passive tracers

@@ -483,7 +483,7 @@ def step(dp: DeviceProblem, redi: OceanRedi, nsteps: int = 1, stream=None) -> No
 
 
 # ---------------------------------------------------------------------------
-# Many domains in one persistent launch (no counterpart in the reference)
+# Many domains in one step (no counterpart in the reference)
 # ---------------------------------------------------------------------------
 STATUS_TIMEOUT = 1
 BATCH_AUTO, BATCH_PERSISTENT, BATCH_LAUNCHES = 0, 1, 2
