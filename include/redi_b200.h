@@ -454,8 +454,10 @@ REDI_B200_API int redi_b200_batch_set_accounting(redi_b200_batch* b, int on);
 REDI_B200_API int redi_b200_batch_stage_times(const redi_b200_batch* b, double* wait_ms, double* busy_ms,
                                               long long* tiles);
 
-/* Longest time a tile waits for its predecessors, or the gate of a step made of
- * launches for a held domain, in ns (default 2e9). */
+/* Longest time a held domain's first tiles, or the gate of a step made of
+ * launches, wait for its release, in ns (default 2e9). A tile waits for its
+ * predecessors a sixteenth longer and 50 us, so that the status names the held
+ * domain's own stage. */
 REDI_B200_API int redi_b200_batch_set_wait_limit(redi_b200_batch* b, long long ns);
 
 /* Fault injection for tests: hold != 0 keeps the domain's first stage waiting

@@ -172,8 +172,11 @@ __global__ void __launch_bounds__(kThreads, OCC) k_domains(const DomainDev<P>* _
                 if (it.stage == S_COLUMN) {
                     ok = wait_released(held + it.domain, &ctl->status, limit_ns);
                 } else {
+                    // blocks claim the stages of a small queue at almost the same time: a little longer than
+                    // for a held domain's release, so that the status names what everything else waits for
                     ok = wait_at_least(&done[it.domain * kMaxStages + it.stage - 1],
-                                       doms[it.domain].ntiles[it.stage - 1], &ctl->status, limit_ns);
+                                       doms[it.domain].ntiles[it.stage - 1], &ctl->status,
+                                       limit_ns + limit_ns / 16 + 50000);
                 }
                 if (ok) {
                     __threadfence();  // the predecessors' writes before this block's reads

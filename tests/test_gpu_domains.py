@@ -400,3 +400,23 @@ def test_persistent_kernel_times_out_and_recovers(redi_lib, precision):
         ref = _handle_run(R, p, 1 if k == 3 else 2, precision)
         for n, (t, c) in enumerate(zip(dp.ms.tracers, ref)):
             _assert_exact(f"{p.name} tracer {n}", t.cpu().numpy(), c)
+
+
+def test_timeout_names_the_held_stage(redi_lib):
+    """All stages of a small batch are claimed at almost the same time; the status names the held domain's
+    column state every time, not a stage that waits behind it."""
+    R = redi_lib
+    ps = _domains()
+    dps = [R.to_device(p) for p in ps]
+    b = R.RediBatch(dps)
+    b.set_form(R.BATCH_PERSISTENT)
+    b.set_wait_limit(2_000_000)  # 2 ms
+    for k in range(40):
+        b.hold(k % len(ps))
+        b.step()
+        st = b.status()
+        assert st["status"] == R.STATUS_TIMEOUT and st["domain"] == k % len(ps) and st["stage"] == 0, (k, st)
+        b.hold(k % len(ps), False)
+    b.step()
+    assert b.status()["status"] == 0
+    b.destroy()
