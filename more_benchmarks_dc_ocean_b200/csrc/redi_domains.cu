@@ -426,8 +426,9 @@ bool prefer_persistent(int nodes, int pairs, double cost) {
     return 1400.0 * nodes > 6.0e4 + 5.2e4 * pairs + 0.08 * cost;
 }
 
+// lean: no byte beyond what the phases need in turn.
 template <class P>
-int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
+int build(redi_b200_batch* b, int n, const redi_b200_domain* dom, bool lean) {
     using Ko = typename P::Ko;
     using He = typename P::He;
     b->host_doms.assign(sizeof(DomainDev<P>) * n, 0);
@@ -468,7 +469,7 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
         const size_t rb = redi::recon_bytes<P>(nx, ny, nz, ntr), fb = redi::flux_bytes<P>(nx, ny, nz, 2);
         // What the two phases need in turn (Phase A's state shares the bytes of Phase B's buffers), and with the
         // fluxes of T and S inside the sweep, where both live at a time: more only for two tracers, by 6 to 9 %
-        // of all that the domain takes. Without room for that the phases run in turn.
+        // of all that the domain takes.
         const size_t in_turn = std::max(a_b, up256(rb) + fb);
         LaunchLayout lay{};
         lay.ts_first = D.ms.idx_temperature == 1 && D.ms.idx_salinity == 2   ? 1
@@ -476,15 +477,10 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom) {
                                                                              : 0;
         lay.ppm_ts = up256(redi::eos_is_linear(D.eos.variant) ? ncol * (nz + 1) * sizeof(redi::IfcState) : a_b);
         lay.flux_ts = up256(lay.ppm_ts + 2 * ncol * nz * sizeof(typename P::Ppm));
-        size_t scratch = lay.ts_first ? std::max(in_turn, lay.flux_ts + fb) : in_turn;
+        if (lean && lay.flux_ts + fb > in_turn) lay.ts_first = 0;  // no room: the phases in turn
+        const size_t scratch = lay.ts_first ? std::max(in_turn, lay.flux_ts + fb) : in_turn;
         char* base = nullptr;
         cudaError_t e = cudaMalloc((void**)&base, coef_b + up256(scratch));
-        if (e == cudaErrorMemoryAllocation && scratch > in_turn) {
-            cudaGetLastError();
-            lay.ts_first = 0;
-            scratch = in_turn;
-            e = cudaMalloc((void**)&base, coef_b + up256(scratch));
-        }
         if (e != cudaSuccess) return bfail(REDI_B200_E_NOMEM, std::string("redi_b200_batch_create: ") + cudaGetErrorString(e));
         const size_t rest = ntr > 2 ? up256(redi::recon_bytes<P>(nx, ny, nz, ntr - 2)) : 0;
         lay.slots = 2 * std::min(redi::kPairsPerLaunch, (ntr - 1) / 2);
@@ -734,23 +730,28 @@ int redi_b200_batch_create(int ndomains, const redi_b200_domain* domains, int pr
     if (tile_bx < 1 || tile_by < 1 || tile_bx * tile_by != kThreads)
         return bfail(REDI_B200_E_ARG, "redi_b200_batch_create: the gather tile must hold 128 cells");
     if (chunk != 4 && chunk != 8 && chunk != 16) return bfail(REDI_B200_E_ARG, "redi_b200_batch_create: chunk must be 4, 8 or 16");
-    redi_b200_batch* b = new (std::nothrow) redi_b200_batch();
-    if (!b) return bfail(REDI_B200_E_NOMEM, "redi_b200_batch_create: host allocation failed");
-    b->precision = precision;
-    b->ndomains = ndomains;
-    b->bx = tile_bx;
-    b->by = tile_by;
-    b->chunk = chunk;
-    b->use_graph = use_graph != 0;
-    const int rc = precision == REDI_B200_MIXED ? build<redi::MixedPrec>(b, ndomains, domains)
-                                                : build<redi::PlainPrec>(b, ndomains, domains);
-    if (rc < 0) {
+    int rc = REDI_B200_OK;
+    for (bool lean : {false, true}) {
+        redi_b200_batch* b = new (std::nothrow) redi_b200_batch();
+        if (!b) return bfail(REDI_B200_E_NOMEM, "redi_b200_batch_create: host allocation failed");
+        b->precision = precision;
+        b->ndomains = ndomains;
+        b->bx = tile_bx;
+        b->by = tile_by;
+        b->chunk = chunk;
+        b->use_graph = use_graph != 0;
+        rc = precision == REDI_B200_MIXED ? build<redi::MixedPrec>(b, ndomains, domains, lean)
+                                          : build<redi::PlainPrec>(b, ndomains, domains, lean);
+        if (rc >= 0) {
+            *out = b;
+            return REDI_B200_OK;
+        }
         free_batch(b);
         delete b;
-        return rc;
+        cudaGetLastError();  // a failed allocation is reported here, not by the next launch
+        if (rc != REDI_B200_E_NOMEM) break;
     }
-    *out = b;
-    return REDI_B200_OK;
+    return rc;
 }
 
 int redi_b200_batch_step(redi_b200_batch* b, void* stream) {

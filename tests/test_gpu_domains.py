@@ -420,3 +420,36 @@ def test_timeout_names_the_held_stage(redi_lib):
     b.step()
     assert b.status()["status"] == 0
     b.destroy()
+
+
+def test_batch_fits_where_the_phases_in_turn_fit(redi_lib):
+    """With room for a little more than the phases in turn, a batch of T and S alone is created without the
+    bytes that its launches would take beyond them, and its step is the handle's."""
+    R = redi_lib
+    b = R.RediBatch([R.to_device(inputs.make_problem(12, 10, 4, seed=3))])  # the kernels are loaded
+    b.step()
+    b.destroy()
+    p, n, mib = inputs.make_problem(200, 200, 25, seed=3), 30, 1 << 20
+    dps = [R.to_device(p) for _ in range(n)]
+    nx, ny, nz = p.nx, p.ny, p.nz
+    faces, ncol, ns = (nx + 1) * ny + nx * (ny + 1), nx * ny, 2 * nz + 2
+    coef = faces * (ns * 24 + (ns - 1) * 8 + 1)
+    in_turn = 2 * ncol * (8 * (nz + 1) + 32 * nz) + 2 * (ns - 1) * faces * 8
+    need = n * ((coef + in_turn) // (2 * mib) + 2) * 2 * mib + 64 * mib
+    assert n * ncol * 16 * (nz + 1) > 256 * mib  # the state of both scalars beside the layers, less the interface values
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - need, dtype=torch.uint8, device="cuda")
+    try:
+        b = R.RediBatch(dps)
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    b.set_form(R.BATCH_LAUNCHES)
+    b.step()
+    assert b.status()["status"] == 0
+    b.destroy()
+    ref = _handle_run(R, p, 1)
+    for k in (0, n // 2, n - 1):
+        for i, (t, c) in enumerate(zip(dps[k].ms.tracers, ref)):
+            _assert_exact(f"domain {k} tracer {i}", t.cpu().numpy(), c)
