@@ -243,9 +243,10 @@ using redi::domains::kMaxStages;
 using redi::domains::kThreads;
 
 // Where a domain's launches keep their buffers when the sweep evaluates the fluxes
-// of T and S. Its scratch is laid out twice: until those two are gathered it holds
-// Phase A's state, their limited layers and their fluxes; after that the passive
-// tracers' reconstruction and as many slots of fluxes as the same bytes take.
+// of T and S. Its scratch is laid out twice: for the sweep it holds Phase A's state
+// and the limited layers of those two, with their fluxes at its end; after it the
+// passive tracers' reconstruction and, once T and S are gathered, as many slots of
+// fluxes behind it as the same bytes take.
 struct LaunchLayout {
     char* scratch;
     size_t ppm_ts, flux_ts;  // offsets, T and S
@@ -403,6 +404,14 @@ int layout_any(redi_b200_batch* b) {
 // 15.1 on one).
 constexpr int kLanes = 12;
 
+// Tiles of faces that fill the device (four blocks on each of 148 SMs). A domain
+// with fewer gains by as many pairs of passive tracers side by side as there are,
+// and takes bytes for them (7 to 10 % more): domains of 86x92x50 and 105x198x50
+// with 34 tracers take 1.25 and 2.98 ms, with the two pairs of the phases' bytes
+// 1.83 and 3.72. Larger ones would gain 2 to 3 % (12 of up to 512x512x75 with 10
+// tracers 23.1 and 23.7 ms; one of 300x200x50 with 8 by itself 1.72 and 1.90).
+constexpr int kFullTiles = 4 * 148;
+
 // Launches of one domain's step: columns, sweep, gather; with passive tracers
 // their reconstruction, and fluxes (mixed precision: a pair at a time) and
 // gathers of `at_once` pairs.
@@ -476,15 +485,21 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom, bool lean) {
                        : D.ms.idx_temperature == 2 && D.ms.idx_salinity == 1 ? 2
                                                                              : 0;
         lay.ppm_ts = up256(redi::eos_is_linear(D.eos.variant) ? ncol * (nz + 1) * sizeof(redi::IfcState) : a_b);
-        lay.flux_ts = up256(lay.ppm_ts + 2 * ncol * nz * sizeof(typename P::Ppm));
-        if (lean && lay.flux_ts + fb > in_turn) lay.ts_first = 0;  // no room: the phases in turn
-        const size_t scratch = lay.ts_first ? std::max(in_turn, lay.flux_ts + fb) : in_turn;
-        char* base = nullptr;
-        cudaError_t e = cudaMalloc((void**)&base, coef_b + up256(scratch));
-        if (e != cudaSuccess) return bfail(REDI_B200_E_NOMEM, std::string("redi_b200_batch_create: ") + cudaGetErrorString(e));
+        const size_t sweep_b = up256(lay.ppm_ts + 2 * ncol * nz * sizeof(typename P::Ppm)) + up256(fb);
+        if (lean && sweep_b > up256(in_turn)) lay.ts_first = 0;  // no room: the phases in turn
+        size_t scratch = lay.ts_first ? std::max(in_turn, sweep_b) : in_turn;
         const size_t rest = ntr > 2 ? up256(redi::recon_bytes<P>(nx, ny, nz, ntr - 2)) : 0;
         lay.slots = 2 * std::min(redi::kPairsPerLaunch, (ntr - 1) / 2);
-        while (lay.slots > 2 && rest + redi::flux_bytes<P>(nx, ny, nz, lay.slots) > scratch) lay.slots -= 2;
+        const int nuf = (nx - 1) * ny, nvf = nx * (ny - 1), nu_tiles = (nuf + kThreads - 1) / kThreads;
+        const int face_tiles = nu_tiles + (nvf + kThreads - 1) / kThreads;
+        if (lean || face_tiles >= kFullTiles)
+            while (lay.slots > 2 && rest + redi::flux_bytes<P>(nx, ny, nz, lay.slots) > scratch) lay.slots -= 2;
+        if (lay.ts_first && lay.slots) scratch = std::max(scratch, rest + redi::flux_bytes<P>(nx, ny, nz, lay.slots));
+        scratch = up256(scratch);
+        lay.flux_ts = scratch - up256(fb);
+        char* base = nullptr;
+        cudaError_t e = cudaMalloc((void**)&base, coef_b + scratch);
+        if (e != cudaSuccess) return bfail(REDI_B200_E_NOMEM, std::string("redi_b200_batch_create: ") + cudaGetErrorString(e));
         b->allocs.push_back(base);
         cudaMemset(base, 0, coef_b);
         char* q = base;
@@ -543,9 +558,7 @@ int build(redi_b200_batch* b, int n, const redi_b200_domain* dom, bool lean) {
             cg.htr_in[t] = D.ms.hTr[t];
         }
         const int npairs = (ntr + 1) / 2;
-        const int nuf = (nx - 1) * ny, nvf = nx * (ny - 1);
-        d.nu_tiles = (nuf + kThreads - 1) / kThreads;
-        const int face_tiles = d.nu_tiles + (nvf + kThreads - 1) / kThreads;
+        d.nu_tiles = nu_tiles;
         d.nstages = redi::domains::S_PAIR0 + 2 * npairs;
         d.ntiles[redi::domains::S_COLUMN] = (int)((ncol + kThreads - 1) / kThreads);
         d.ntiles[redi::domains::S_SWEEP] = face_tiles;
@@ -652,19 +665,20 @@ cudaError_t enqueue_domain(const DomainDev<P>& d, const LaunchLayout& lay, cudaS
     flux_buffer(ff, cg, lay.scratch + lay.flux_ts, 2, 0, 2);
     e = redi::launch_column_recon<P>(d.cs, rc, swap, form, st);
     if (e == cudaSuccess) e = redi::launch_sweep_flux<P>(d.sw, ff, swap, form, st);
+    redi::ReconArgsT<P> rest = d.rc;
+    rest.ntr = ntr - 2;
+    for (int k = 0; k < rest.ntr; ++k) rest.htr[k] = d.rc.htr[2 + k];
+    rest.ti = reinterpret_cast<double*>(lay.scratch);
+    rest.ppm = reinterpret_cast<typename P::Ppm*>(lay.scratch + redi::recon_ppm_offset(rc.nx, rc.ny, rc.nz, rest.ntr));
+    if (e == cudaSuccess && rest.ntr > 0) e = redi::launch_tracer_recon<P>(rest, st);
     if (e == cudaSuccess) e = redi::launch_phase_b<P>(rc, ff, cg, st, redi::Band{}, 2, 2, true);
-    if (e != cudaSuccess || ntr == 2) return e;
-    rc = d.rc;
+    if (e != cudaSuccess || rest.ntr == 0) return e;
     ff = d.ff;
     cg = d.cg;
-    rc.ntr = ntr - 2;
-    for (int k = 0; k < rc.ntr; ++k) rc.htr[k] = d.rc.htr[2 + k];
-    rc.ti = reinterpret_cast<double*>(lay.scratch);
-    rc.ppm = reinterpret_cast<typename P::Ppm*>(lay.scratch + redi::recon_ppm_offset(rc.nx, rc.ny, rc.nz, rc.ntr));
-    ff.ti = rc.ti;
-    ff.ppm = rc.ppm;
-    flux_buffer(ff, cg, lay.scratch + up256(redi::recon_bytes<P>(rc.nx, rc.ny, rc.nz, rc.ntr)), lay.slots, 2, rc.ntr);
-    return redi::launch_phase_b<P>(rc, ff, cg, st, redi::Band{}, 0, 0, true);
+    ff.ti = rest.ti;
+    ff.ppm = rest.ppm;
+    flux_buffer(ff, cg, lay.scratch + up256(redi::recon_bytes<P>(rc.nx, rc.ny, rc.nz, rest.ntr)), lay.slots, 2, rest.ntr);
+    return redi::launch_phase_b<P>(rest, ff, cg, st, redi::Band{}, rest.ntr, 0, true);
 }
 
 template <class P>

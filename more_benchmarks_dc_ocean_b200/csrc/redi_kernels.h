@@ -342,6 +342,9 @@ cudaError_t launch_eos_points(const EosParams& e, int n, const double* T, const 
                               double* rho, double* dsv_dt, double* dsv_ds, cudaStream_t st);
 template <class P>
 cudaError_t launch_sweep(const SweepArgsT<P>& sw, cudaStream_t st, Band band = Band{});
+// The reconstruction of rc's tracers, as launch_phase_b runs it.
+template <class P>
+cudaError_t launch_tracer_recon(const ReconArgsT<P>& rc, cudaStream_t st);
 // recon_from: the first tracer of rc to reconstruct (tracers before it were
 // reconstructed already, by launch_column_recon). flux_from: 2 when the fluxes
 // of tracers 0 and 1 are in flux slots 0 and 1 already (launch_sweep_flux).

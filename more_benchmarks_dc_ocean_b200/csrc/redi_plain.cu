@@ -592,6 +592,14 @@ void launch_recon(const ReconArgsT<P>& rc, const BandRanges& r, cudaStream_t st)
     launch_end(kid, st);
 }
 
+template <class P>
+cudaError_t launch_tracer_recon(const ReconArgsT<P>& rc, cudaStream_t st) {
+    launch_recon<P>(rc, band_ranges(rc.nx, rc.ny, Band{}), st);
+    return cudaGetLastError();
+}
+template cudaError_t launch_tracer_recon<PlainPrec>(const ReconArgsT<PlainPrec>&, cudaStream_t);
+template cudaError_t launch_tracer_recon<MixedPrec>(const ReconArgsT<MixedPrec>&, cudaStream_t);
+
 // ---------------------------------------------------------------------------
 // The fused face-flux + fold pass (redi_fold.cuh).
 // ---------------------------------------------------------------------------
